@@ -1,0 +1,60 @@
+"""The device-wide primitives against numpy (needs a GB300): compiled with a small host
+entry of their own, since the C ABI does not export them."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from acvd_gb300 import build
+
+pytestmark = pytest.mark.gpu
+
+HARNESS = r"""
+#include "%s/primitives.cu"
+template <class T> struct Dev {
+    T* p = nullptr;
+    Dev(const T* h, size_t n) {
+        cudaMalloc((void**)&p, (n + 1) * sizeof(T));
+        if (h) cudaMemcpy(p, h, n * sizeof(T), cudaMemcpyHostToDevice);
+    }
+    ~Dev() { cudaFree(p); }
+};
+extern "C" int test_sort(unsigned* keys, unsigned* vals, long long n, int bits) {
+    Dev<unsigned> k(keys, n), v(vals, n), tk(nullptr, n), tv(nullptr, n);
+    acvd::Scratch sc;
+    if (acvd::radix_sort_pairs(k.p, v.p, tk.p, tv.p, n, bits, sc, 0) != cudaSuccess) return 1;
+    cudaMemcpy(keys, k.p, n * 4, cudaMemcpyDeviceToHost);
+    cudaMemcpy(vals, v.p, n * 4, cudaMemcpyDeviceToHost);
+    return (int)cudaDeviceSynchronize();
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    d = tmp_path_factory.mktemp("prim")
+    src, so = d / "harness.cu", d / "harness.so"
+    src.write_text(HARNESS % build.SRC)
+    subprocess.run([build._nvcc(), build.ARCH, "-O3", "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "-o", str(so),
+                    str(src), "-lcudart"], check=True, capture_output=True)
+    return ctypes.CDLL(str(so))
+
+
+# the edges of the tiles (1,024 and 2,048 pairs), of the short form (512 tiles of 1,024) and of
+# the row scan (1,024 tiles), for 1 to 4 passes of 8 bits and 2 and 3 of 10
+@pytest.mark.parametrize("n", [2, 31, 1023, 1024, 1025, 2049, 4097, 524287, 524289, 2100003])
+@pytest.mark.parametrize("bits", [1, 8, 15, 17, 20, 24, 26, 32])
+def test_radix_sort_is_stable(lib, n, bits):
+    rng = np.random.default_rng(n + bits)
+    keys = rng.integers(0, 1 << bits, n, dtype=np.uint64).astype(np.uint32)
+    if n % 2:   # few distinct keys: long runs of equal digits
+        keys = keys[rng.integers(0, min(n, 5), n)]
+    vals = np.arange(n, dtype=np.uint32)
+    order = np.argsort(keys, kind="stable")
+    k, v = keys.copy(), vals.copy()
+    P = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    assert lib.test_sort(P(k), P(v), ctypes.c_longlong(n), bits) == 0
+    np.testing.assert_array_equal(k, keys[order])
+    np.testing.assert_array_equal(v, vals[order])

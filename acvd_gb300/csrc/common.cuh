@@ -146,6 +146,49 @@ ACVD_DEV unsigned prio_of_delta(float dE) {
 }
 
 // ---------------------------------------------------------------------------
+// Correctly rounded float32 square root and reciprocal without the range checks and
+// slow path of the general ones, for arguments in [1, 2^82]: the hardware's approximation,
+// then one Newton step in FMA form on the residual, which is exact (Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", 1990).  Both equal the
+// IEEE operation for every significand (and, the root, both parities of the exponent):
+// neither step leaves the normal range here, so the exponent only scales them.
+// ---------------------------------------------------------------------------
+ACVD_DEV float root_rn(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    const float s = __fmul_rn(x, y);
+    return __fmaf_rn(__fmaf_rn(-s, s, x), __fmul_rn(0.5f, y), s);
+}
+
+ACVD_DEV float recip_rn(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
+}
+
+// Tangent and cosine of the Jacobi rotation of cotangent 2 theta: t = sign(theta) /
+// (|theta| + sqrt(theta^2 + 1)), c = 1 / sqrt(t^2 + 1).
+ACVD_DEV void jacobi_rotation(double theta, double& t, double& c) {
+    t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+    c = 1.0 / sqrt(t * t + 1.0);
+}
+
+// The float32 form bounds the energy tests: five dependent roots and quotients per
+// rotation, about twelve rotations per test.  The same bits as the general operations,
+// which stay for |theta| >= 2^40 (where theta^2 may overflow) and NaN.
+ACVD_DEV void jacobi_rotation(float theta, float& t, float& c) {
+    const float a = fabsf(theta);
+    if (a < 0x1p40f) {
+        const float r = recip_rn(__fadd_rn(a, root_rn(__fmaf_rn(theta, theta, 1.0f))));
+        t = theta >= 0.0f ? r : -r;
+        c = recip_rn(root_rn(__fmaf_rn(t, t, 1.0f)));
+        return;
+    }
+    t = (theta >= 0.0f ? 1.0f : -1.0f) / (a + sqrtf(theta * theta + 1.0f));
+    c = 1.0f / sqrtf(t * t + 1.0f);
+}
+
+// ---------------------------------------------------------------------------
 // Small symmetric 3x3 eigen-solver by cyclic Jacobi rotations (Jacobi 1846;
 // Golub & Van Loan, Matrix Computations, sec. 8.5).  a = {a00,a01,a02,a11,a12,a22}.
 // On return w holds the eigenvalues and V (columns) the eigenvectors.
@@ -169,8 +212,8 @@ ACVD_DEV void jacobi_eig3(const T a6[6], T w[3], T V[3][3], int max_sweeps) {
             const T apq = A[p][q];
             if (apq == T(0)) continue;
             const T theta = (A[q][q] - A[p][p]) / (T(2) * apq);
-            const T t = (theta >= T(0) ? T(1) : T(-1)) / (fabs(theta) + sqrt(theta * theta + T(1)));
-            const T c = T(1) / sqrt(t * t + T(1));
+            T t, c;
+            jacobi_rotation(theta, t, c);
             const T sn = t * c;
 #pragma unroll
             for (int k = 0; k < 3; k++) {

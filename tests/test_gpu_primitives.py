@@ -29,6 +29,29 @@ extern "C" int test_sort(unsigned* keys, unsigned* vals, long long n, int bits) 
     cudaMemcpy(vals, v.p, n * 4, cudaMemcpyDeviceToHost);
     return (int)cudaDeviceSynchronize();
 }
+// the short roots and reciprocals against the IEEE operations: counts of differing bits
+__global__ void roots_kernel(unsigned long long* bad) {
+    const unsigned step = gridDim.x * blockDim.x;
+    for (unsigned m = blockIdx.x * blockDim.x + threadIdx.x; m < (1u << 24); m += step) {
+        // every significand, exponents 0 and 1, then the same far up the range
+        for (int e = 0; e <= 80; e += 16) {
+            const float x = ldexpf(__uint_as_float(0x3f800000u + m), e);
+            if (acvd::root_rn(x) != __fsqrt_rn(x)) atomicAdd(&bad[0], 1ull);
+            if (acvd::recip_rn(x) != __frcp_rn(x)) atomicAdd(&bad[1], 1ull);
+        }
+        // t^2 + 1 lies in [1, 2]
+        const float u = 1.0f + (float)m * 0x1p-24f;
+        if (acvd::recip_rn(acvd::root_rn(u)) != __frcp_rn(__fsqrt_rn(u))) atomicAdd(&bad[2], 1ull);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        if (acvd::recip_rn(acvd::root_rn(2.0f)) != __frcp_rn(__fsqrt_rn(2.0f))) atomicAdd(&bad[2], 1ull);
+}
+extern "C" int test_roots(unsigned long long* bad) {
+    Dev<unsigned long long> d(bad, 3);
+    roots_kernel<<<2048, 256>>>(d.p);
+    cudaMemcpy(bad, d.p, 24, cudaMemcpyDeviceToHost);
+    return (int)cudaDeviceSynchronize();
+}
 """
 
 
@@ -58,3 +81,9 @@ def test_radix_sort_is_stable(lib, n, bits):
     assert lib.test_sort(P(k), P(v), ctypes.c_longlong(n), bits) == 0
     np.testing.assert_array_equal(k, keys[order])
     np.testing.assert_array_equal(v, vals[order])
+
+
+def test_short_roots_and_reciprocals_are_correctly_rounded(lib):
+    bad = np.zeros(3, dtype=np.uint64)
+    assert lib.test_roots(bad.ctypes.data_as(ctypes.c_void_p)) == 0
+    np.testing.assert_array_equal(bad, 0)

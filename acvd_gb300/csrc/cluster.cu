@@ -298,8 +298,7 @@ ACVD_DEV void set_cached_ev(const DevState& st, int i, int4 c, int ev) {
 }
 
 template <int M, int TB = 256>
-ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
-                        int* cand_dest, unsigned* cand_prio, int claims, int64_t tile,
+ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color, int claims, int64_t tile,
                         const int* entries = nullptr, int n_entries = 0) {
     __shared__ int s_idx[TB];                 // work item -> colour-list position
     __shared__ int s_tgt[TB][kMaxTgt];        // work item -> destination clusters (ring order)
@@ -541,7 +540,7 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
     }
     __syncthreads();
     // B2: decision
-    int my_cand = -1;
+    int4 my_cand = make_int4(-1, -1, -1, 0);   // x = -1: no proposal
     if (threadIdx.x < s_nwork) {
         const int w = threadIdx.x;
         const int widx = s_idx[w];
@@ -606,8 +605,6 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
             }
         }
         if (best >= 0) {
-            cand_dest[widx] = best;
-            cand_prio[widx] = pr;
             if (claims) {
                 const unsigned long long c = make_claim((unsigned)epoch, pr, (unsigned)widx);
                 if (L < st.k) atomicMin(&st.claim[L], c);
@@ -616,7 +613,7 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
                 atomicAdd(&st.out_cnt[L], 1);   // relaxed step: proposals leaving L
             }
             n_cand = 1;
-            my_cand = widx;
+            my_cand = make_int4(widx, best, L, (int)pr);
             st.evald[i] = -1;
             if (s_rec[w]) set_cached_ev(st, i, st.tcache[i], -1);
         } else {
@@ -632,7 +629,7 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
         constexpr int kW = TB / 32;
         __shared__ unsigned s_wc[kW], s_base, s_cnt[kW][kNC];
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        const unsigned bal = __ballot_sync(kFull, my_cand >= 0);
+        const unsigned bal = __ballot_sync(kFull, my_cand.x >= 0);
         const unsigned v[kNC] = {(in && !listed) ? 1u : 0u, n_scr - n_cached, n_cached, n_slots, n_bnd, n_tgt,
                                  n_cand};
 #pragma unroll
@@ -659,7 +656,7 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
             if (t) atomicAdd(ctr(st.counters, which), (unsigned long long)t);
         }
         __syncthreads();
-        if (my_cand >= 0) st.cand_list[s_base + s_wc[wid] + __popc(bal & ((1u << lane) - 1u))] = my_cand;
+        if (my_cand.x >= 0) st.cand_list[s_base + s_wc[wid] + __popc(bal & ((1u << lane) - 1u))] = my_cand;
     }
 }
 
@@ -674,8 +671,8 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
 // let more of them be in different phases of their tiles.
 template <int M, int B, int TB = 256>
 __global__ void __launch_bounds__(TB, B * 256 / TB) eval_kernel(DevState st, int item0, int64_t count, int color,
-                                                                int* cand_dest, unsigned* cand_prio, int claims) {
-    eval_tile<M, TB>(st, item0, count, color, cand_dest, cand_prio, claims, blockIdx.x);
+                                                                int claims) {
+    eval_tile<M, TB>(st, item0, count, color, claims, blockIdx.x);
 }
 
 // default blocks per SM: the fused evaluation 4 (isotropic, QEM) and 5 (the
@@ -815,8 +812,7 @@ __global__ void __launch_bounds__(256, 4) screen_kernel(DevState st, int item0, 
 // grid-stride over (stripe, tile) pairs.
 template <int M, int B, int TB = 256>
 __global__ void __launch_bounds__(TB, B * 256 / TB) eval_list_kernel(DevState st, int item0, int64_t count,
-                                                                     int color, int* cand_dest, unsigned* cand_prio,
-                                                                     int claims, const int* work,
+                                                                     int color, int claims, const int* work,
                                                                      const unsigned* work_count) {
     __shared__ unsigned s_cnt[kWorkStripes];
     if (threadIdx.x < kWorkStripes) s_cnt[threadIdx.x] = work_count[color * kWorkStripes + threadIdx.x];
@@ -830,7 +826,7 @@ __global__ void __launch_bounds__(TB, B * 256 / TB) eval_list_kernel(DevState st
         const int64_t j = t / kWorkStripes;
         const int64_t have = (int64_t)s_cnt[q] - j * TB;
         if (have <= 0) continue;   // block-uniform
-        eval_tile<M, TB>(st, item0, count, color, cand_dest, cand_prio, claims, t, work + q * cap + j * TB,
+        eval_tile<M, TB>(st, item0, count, color, claims, t, work + q * cap + j * TB,
                          have < TB ? (int)have : TB);
     }
 }
@@ -1029,43 +1025,131 @@ ACVD_DEV void update_cluster(const DevState& st, int k) {
 }
 
 // ---------------------------------------------------------------------------
-// apply: commit the proposals that hold both claims (grid-stride over the
-// step's compact proposal list)
+// Committing a step's proposals.  The list's length is known on the device only, and it
+// is short next to the class: 5 to 10,000 proposals.  Both commit kernels are a chain of
+// dependent loads and one record update per proposal, so they give a proposal to a lane
+// (pair) of warp j % W, W the grid's warps: a short list spreads over every SM, one or two
+// proposals to a warp.  (With consecutive proposals in one block of 256, a list of 4,800 ran
+// on 19 SMs: 8-11 us a launch at the 1024 x 512 torus.)  A proposal's record carries its
+// clusters and priority, and is read beside the length, so that only one load separates the
+// launch from the clusters' records.
 // ---------------------------------------------------------------------------
-// gtid / gstride: this thread's position and the number of threads walking the
-// list.  A lane pair handles one proposal: the even lane the destination
-// cluster B, the odd lane the source cluster L; the pair exchanges the two new
-// energies and both take the same decision.
+constexpr int kCommitThreads = 128;
+constexpr int kCommitWarps = kCommitThreads / 32;
+
+// A load issued here, not sunk to where its value is used (behind a branch that most of
+// the loads' latency would then follow).
+ACVD_DEV float2 load_now(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+ACVD_DEV float4 load_now(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+ACVD_DEV int4 load_now(const int4* p) {
+    int4 v;
+    asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+ACVD_DEV int load_now(const int* p) {
+    int v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+ACVD_DEV double load_now(const double* p) {
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
 template <int M>
-ACVD_DEV void apply_range(const DevState& st, int item0, int color, int round, int* cand_dest,
-                          const unsigned* cand_prio, unsigned gtid, unsigned gstride) {
+ACVD_DEV void load_item_now(const DevState& st, int i, ItemRec& it) {
+    const float4 a = load_now(st.xw + i);
+    it.x[0] = a.x; it.x[1] = a.y; it.x[2] = a.z; it.w = a.w;
+    if (M != kIso) {
+        const float4 q = load_now(st.qa + i);
+        const float2 r = load_now(st.qb + i);
+        it.A[0] = q.x; it.A[1] = q.y; it.A[2] = q.z; it.A[3] = q.w; it.A[4] = r.x; it.A[5] = r.y;
+    }
+    if (M == kAniso) {
+        const float4 t = load_now(st.ta + i);
+        const float2 u = load_now(st.tb + i);
+        it.T[0] = t.x; it.T[1] = t.y; it.T[2] = t.z; it.T[3] = t.w; it.T[4] = u.x; it.T[5] = u.y;
+    }
+}
+
+// mark_ring with the first 8 neighbours already loaded
+ACVD_DEV void mark_ring8(const DevState& st, int i, int4 a, int4 b) {
+    if (b.w == -2) {   // a longer ring
+        mark_ring(st, i);
+        return;
+    }
+    st.bflag[i] = 1;
+    const int nb[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+        if (nb[q] >= 0) st.bflag[nb[q]] = 1;
+}
+
+// ---------------------------------------------------------------------------
+// apply: commit the proposals that hold both claims.  warp / nwarps: this warp's
+// position among those that walk the list (count: the class's items, the list's
+// capacity).  A lane pair handles one proposal: the even lane the destination
+// cluster B, the odd lane the source cluster L; the pair exchanges the two new
+// energies and both take the same decision.  The records a winner updates are loaded
+// with the claims that decide whether it wins.
+// ---------------------------------------------------------------------------
+template <int M>
+ACVD_DEV void apply_range(const DevState& st, int item0, int64_t count, int color, int round, unsigned warp,
+                          unsigned nwarps) {
+    constexpr int NA = Layout<M>::acc;
+    const unsigned lane = threadIdx.x & 31u;
+    const int role = (int)(lane & 1u);
+    const unsigned pair_mask = 3u << (lane & ~1u);
+    unsigned j = warp + (lane >> 1) * nwarps;
+    int4 e = j < (unsigned)count ? load_now(st.cand_list + j) : make_int4(0, -1, 0, 0);
     const unsigned n = st.cand_count[color];
     const unsigned epoch = (unsigned)(color * kRounds + round);
-    const int role = (int)(gtid & 1u);
-    const unsigned pair_mask = 3u << ((threadIdx.x & 31u) & ~1u);
     unsigned won_total = 0;
-    for (unsigned j = gtid >> 1; j < n; j += gstride >> 1) {
-        const int idx = st.cand_list[j];
-        const int B = cand_dest[idx];
+    while (j < n) {
+        const unsigned at = j;
+        const int idx = e.x, B = e.y, L = e.z;
+        const unsigned prio = (unsigned)e.w;
+        j += 16u * nwarps;
+        if (j < n) e = st.cand_list[j];
         if (B < 0) continue;                     // committed or dropped in an earlier round
-        const int i = item0 + (int)idx;
-        const int L = st.label[i];
-        if (!ACVD_VALID(st, B < st.k && L >= 0 && L <= st.k)) continue;
-        const unsigned long long key = make_claim(epoch, cand_prio[idx], (unsigned)idx);
-        if (st.claim[B] != key || (L < st.k && st.claim[L] != key)) continue;
-        __syncwarp(pair_mask);                   // both lanes have read the claims and cand_dest
+        const int i = item0 + idx;
+        if (!ACVD_VALID(st, B < st.k && L >= 0 && L <= st.k && L == st.label[i])) continue;
+        const unsigned long long key = make_claim(epoch, prio, (unsigned)idx);
+        const int C = role && L < st.k ? L : B;  // the cluster of this lane
+        const unsigned long long claim_b = st.claim[B], claim_l = st.claim[L < st.k ? L : B];
         ItemRec it;
-        load_item<M>(st, i, it);
+        load_item_now<M>(st, i, it);
+        const int4 ra = load_now(st.ring8 + 2 * (int64_t)i), rb = load_now(st.ring8 + 2 * (int64_t)i + 1);
+        df* aC = st.acc + (int64_t)C * NA;
+        const double e_mine = load_now(st.energy + C);
+        const int size = load_now(st.size + C);
+        df nC[NA];
+#pragma unroll
+        for (int q = 0; q < NA; q++) {
+            const float2 v = load_now(reinterpret_cast<const float2*>(aC) + q);
+            nC[q] = {v.x, v.y};
+        }
+        if (claim_b != key || (L < st.k && claim_l != key)) continue;
+        __syncwarp(pair_mask);                   // both lanes have read the claims and the proposal
         const int now = st.sweep->sweep;
         if (L >= st.k) {
             // unassigned item joining a cluster: always committed
             if (role == 0) {
                 st.claim[B] = claim_taken(color);   // taken for the rest of this step
-                cand_dest[idx] = -1;
+                st.cand_list[at].y = -1;
                 won_total++;
                 st.label[i] = B;
-                mark_ring(st, i);
-                st.size[B] += 1;
+                mark_ring8(st, i, ra, rb);
+                st.size[B] = size + 1;
                 st.stamp[B] = now;
                 accumulate_item<M>(st.acc + (int64_t)B * Layout<M>::acc, it, 1.0f);
                 update_cluster<M, false>(st, B);
@@ -1076,14 +1160,8 @@ ACVD_DEV void apply_range(const DevState& st, int item0, int color, int round, i
         // energy of the pair strictly decreases (the float32 test can disagree with
         // the updated records, e.g. when a pseudo-inverse eigenvalue sits at the
         // threshold), so the minimisation descends monotonically and terminates
-        const int C = role ? L : B;
-        df* aC = st.acc + (int64_t)C * Layout<M>::acc;
         float4* eC = st.ev + (int64_t)C * Layout<M>::ev;
         const RunFlags fl = *st.flags;
-        const double e_mine = st.energy[C];
-        df nC[Layout<M>::acc];
-#pragma unroll
-        for (int q = 0; q < Layout<M>::acc; q++) nC[q] = aC[q];
         accumulate_item<M>(nC, it, role ? -1.0f : 1.0f);
         float4 rC[Layout<M>::ev];
         const int anc = anchor_of<M>(st, C);
@@ -1096,23 +1174,23 @@ ACVD_DEV void apply_range(const DevState& st, int item0, int color, int round, i
         const double e_new = role ? en_other + en_mine : en_mine + en_other;
         if (e_new < e_old) {
 #pragma unroll
-            for (int q = 0; q < Layout<M>::acc; q++) aC[q] = nC[q];
+            for (int q = 0; q < NA; q++) aC[q] = nC[q];
 #pragma unroll
             for (int q = 0; q < Layout<M>::ev; q++) eC[q] = rC[q];
             st.energy[C] = en_mine;
-            st.size[C] += role ? -1 : 1;
+            st.size[C] = size + (role ? -1 : 1);
             st.stamp[C] = now;
             st.claim[C] = claim_taken(color);   // taken for the rest of this step
             if (role == 0) {
                 won_total++;
                 st.label[i] = B;
-                mark_ring(st, i);
-                cand_dest[idx] = -1;
+                mark_ring8(st, i, ra, rb);
+                st.cand_list[at].y = -1;
             }
         } else {
             st.claim[C] = claim_taken(color);
             if (role == 0) {
-                cand_dest[idx] = -1;
+                st.cand_list[at].y = -1;
                 atomicAdd(ctr(st.counters, kCntReverted), 1ull);
             }
         }
@@ -1122,40 +1200,36 @@ ACVD_DEV void apply_range(const DevState& st, int item0, int color, int round, i
 }
 
 template <int M>
-__global__ void __launch_bounds__(256) apply_kernel(DevState st, int item0, int color,
-                                                    int round, int* cand_dest, const unsigned* cand_prio) {
-    apply_range<M>(st, item0, color, round, cand_dest, cand_prio, blockIdx.x * blockDim.x + threadIdx.x,
-                   gridDim.x * blockDim.x);
+__global__ void __launch_bounds__(kCommitThreads) apply_kernel(DevState st, int item0, int64_t count, int color,
+                                                               int round) {
+    apply_range<M>(st, item0, count, color, round, blockIdx.x * kCommitWarps + (threadIdx.x >> 5),
+                   gridDim.x * kCommitWarps);
 }
 
 // Next matching round of a step: a proposal whose two clusters were not touched
 // by this step's commits still carries an exact energy change and claims again
 // with a newer epoch; one that lost a cluster to a commit is dropped (its item
 // is evaluated again next sweep).
-ACVD_DEV void reclaim_range(const DevState& st, int item0, int color, int round, int* cand_dest,
-                            const unsigned* cand_prio, unsigned gtid, unsigned gstride) {
+ACVD_DEV void reclaim_range(const DevState& st, int item0, int color, int round, unsigned gtid, unsigned gstride) {
     const unsigned n = st.cand_count[color];
     const unsigned epoch = (unsigned)(color * kRounds + round);
     for (unsigned j = gtid; j < n; j += gstride) {
-        const int idx = st.cand_list[j];
-        const int B = cand_dest[idx];
+        const int4 e = st.cand_list[j];
+        const int B = e.y, L = e.z;
         if (B < 0) continue;
-        const int L = st.label[item0 + idx];
         const unsigned long long taken = claim_taken(color);
         if (st.claim[B] == taken || (L < st.k && st.claim[L] == taken)) {
-            cand_dest[idx] = -1;
+            st.cand_list[j].y = -1;
             continue;
         }
-        const unsigned long long key = make_claim(epoch, cand_prio[idx], (unsigned)idx);
+        const unsigned long long key = make_claim(epoch, (unsigned)e.w, (unsigned)e.x);
         if (L < st.k) atomicMin(&st.claim[L], key);
         atomicMin(&st.claim[B], key);
     }
 }
 
-__global__ void reclaim_kernel(DevState st, int item0, int color, int round, int* cand_dest,
-                               const unsigned* cand_prio) {
-    reclaim_range(st, item0, color, round, cand_dest, cand_prio, blockIdx.x * blockDim.x + threadIdx.x,
-                  gridDim.x * blockDim.x);
+__global__ void reclaim_kernel(DevState st, int item0, int color, int round) {
+    reclaim_range(st, item0, color, round, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1199,49 +1273,96 @@ ACVD_DEV df from_fixed(long long d, float4 p) {
     return df_renorm(__fmul_rn(__fmul_rn(h, p.z), p.w), __fmul_rn(__fmul_rn(l, p.z), p.w));
 }
 
+// The fixed-point sums of a proposal, added by a group of lanes: its contributions are
+// staged in shared memory (lane p's proposal in s_v[p]), then GROUP lanes add the
+// components of one cluster side by side, so that the atomics of a cluster fall in one or
+// two 128-byte lines instead of one each.
 template <int M>
-ACVD_DEV void relaxed_commit_range(const DevState& st, int item0, int color,
-                                   const int* cand_dest, unsigned gtid, unsigned gstride) {
+struct CommitStage {
+    static constexpr int NA = Layout<M>::acc;
+    static constexpr int GROUP = M == kIso ? 4 : (M == kQEM ? 16 : 32);
+    long long v[32][NA];
+    int cl[32][2];   // destination and source; -1: none
+};
+
+template <int M>
+ACVD_DEV void relaxed_commit_range(const DevState& st, int item0, int64_t count, int color, unsigned warp,
+                                   unsigned nwarps, CommitStage<M>& s) {
     constexpr int NA = Layout<M>::acc;
+    constexpr int GROUP = CommitStage<M>::GROUP;
+    const unsigned lane = threadIdx.x & 31u;
+    // up to 32 proposals per warp: lane l takes proposal warp + l * nwarps; longer lists go
+    // by runs of 32 consecutive proposals, whose items lie near one another
+    unsigned j = warp + lane * nwarps;
+    int4 e = j < (unsigned)count ? load_now(st.cand_list + j) : make_int4(0, 0, 0, 0);
     const unsigned n = st.cand_count[color];
+    const bool runs = n > 32u * nwarps;
+    const unsigned step = 32u * nwarps;
+    unsigned first = warp;                        // lane 0's proposal
+    if (runs) {
+        first = warp * 32u;
+        j = first + lane;
+        if (j < n) e = st.cand_list[j];
+    }
     unsigned won = 0;
     const int now = st.sweep->sweep;
-    for (unsigned j = gtid; j < n; j += gstride) {
-        const int idx = st.cand_list[j];
-        const int i = item0 + (int)idx;
-        const int B = cand_dest[idx];
-        const int L = st.label[i];
-        if (!ACVD_VALID(st, B >= 0 && B < st.k && L >= 0 && L <= st.k)) continue;
+    for (; first < n; first += step, j += step) {
+        if (j >= step && j < n) e = st.cand_list[j];
+        bool live = j < n;
+        const int i = item0 + e.x, B = e.y, L = e.z;
+        if (live && !ACVD_VALID(st, B >= 0 && B < st.k && L >= 0 && L <= st.k && L == st.label[i])) live = false;
+        const bool from = live && L < st.k;
+        int4 ra = make_int4(-1, -1, -1, -1), rb = ra;
+        int size = 0, out = 0;
+        ItemRec it;
+        if (live) {
+            load_item_now<M>(st, i, it);
+            ra = load_now(st.ring8 + 2 * (int64_t)i);
+            rb = load_now(st.ring8 + 2 * (int64_t)i + 1);
+            if (from) {
+                size = load_now(st.size + L);
+                out = load_now(st.out_cnt + L);
+            }
+        }
         // sizes are untouched until fx_finalize: a cluster whose every member would
         // leave keeps them all
-        if (L < st.k && st.size[L] - st.out_cnt[L] < 1) continue;
-        won++;
-        ItemRec it;
-        load_item<M>(st, i, it);
-        st.label[i] = B;
-        mark_ring(st, i);
-        atomicAdd(&st.in_done[B], 1);
-        st.stamp[B] = now;
-        long long* dB = st.fx_delta + (int64_t)B * NA;
-        long long* dL = st.fx_delta + (int64_t)(L < st.k ? L : 0) * NA;
-        if (L < st.k) {
-            atomicAdd(&st.out_done[L], 1);
-            st.stamp[L] = now;
-        }
+        if (from && size - out < 1) live = false;
+        s.cl[lane][0] = live ? B : -1;
+        s.cl[lane][1] = live && from ? L : -1;
+        if (live) {
+            won++;
+            st.label[i] = B;
+            mark_ring8(st, i, ra, rb);
+            atomicAdd(&st.in_done[B], 1);
+            st.stamp[B] = now;
+            if (from) {
+                atomicAdd(&st.out_done[L], 1);
+                st.stamp[L] = now;
+            }
 #pragma unroll
-        for (int q = 0; q < NA; q++) {
-            const long long v = to_fixed(contrib_df<M>(it, q), st.fx_pow[q]);
-            atomicAdd((unsigned long long*)&dB[q], (unsigned long long)v);
-            if (L < st.k) atomicAdd((unsigned long long*)&dL[q], (unsigned long long)(-v));
+            for (int q = 0; q < NA; q++) s.v[lane][q] = to_fixed(contrib_df<M>(it, q), st.fx_pow[q]);
         }
+        const unsigned have = 32u - (unsigned)__clz((int)__ballot_sync(kFull, live));   // lanes in use
+        __syncwarp();
+        const unsigned g = lane / GROUP, q = lane % GROUP;
+        for (unsigned t = g; t < 2u * have; t += 32u / GROUP) {
+            const unsigned p = t >> 1, side = t & 1u;
+            const int c = s.cl[p][side];
+            if (c < 0 || q >= (unsigned)NA) continue;
+            const long long v = s.v[p][q];
+            atomicAdd((unsigned long long*)&st.fx_delta[(int64_t)c * NA + q], (unsigned long long)(side ? -v : v));
+        }
+        __syncwarp();
     }
     warp_count(ctr(st.counters, kCntMoves), won);
 }
 
 template <int M>
-__global__ void relaxed_commit_kernel(DevState st, int item0, int color, const int* cand_dest) {
-    relaxed_commit_range<M>(st, item0, color, cand_dest, blockIdx.x * blockDim.x + threadIdx.x,
-                            gridDim.x * blockDim.x);
+__global__ void __launch_bounds__(kCommitThreads) relaxed_commit_kernel(DevState st, int item0, int64_t count,
+                                                                        int color) {
+    __shared__ CommitStage<M> s[kCommitWarps];
+    relaxed_commit_range<M>(st, item0, count, color, blockIdx.x * kCommitWarps + (threadIdx.x >> 5),
+                            gridDim.x * kCommitWarps, s[threadIdx.x >> 5]);
 }
 
 template <int M>
@@ -1418,6 +1539,8 @@ __global__ void __launch_bounds__(256, 2) sweep_run_kernel(SweepRun a) {
     const unsigned gstride = gridDim.x * blockDim.x;
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
     volatile LoopState* vls = a.ls;
+    extern __shared__ __align__(16) char stage_mem[];   // 8 warps' commit stages
+    CommitStage<M>* stage = reinterpret_cast<CommitStage<M>*>(stage_mem);
     for (;;) {
         const bool relaxed = vls->relaxed_ok && !st.flags->connexity;
         if (lead) {
@@ -1438,21 +1561,21 @@ __global__ void __launch_bounds__(256, 2) sweep_run_kernel(SweepRun a) {
             const unsigned long long t0 = lead ? global_ns() : 0ull;
             const int64_t ntiles = (cnt + 255) / 256;
             for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x)
-                eval_tile<M>(st, item0, cnt, c, a.cand_dest, a.cand_prio, relaxed ? 0 : 1, t);
+                eval_tile<M>(st, item0, cnt, c, relaxed ? 0 : 1, t);
             if (!grid_barrier(a.bar)) return;
             if (lead) a.ls->eval_ns += global_ns() - t0;
             if (relaxed) {
-                relaxed_commit_range<M>(st, item0, c, a.cand_dest, gtid, gstride);
+                relaxed_commit_range<M>(st, item0, cnt, c, gtid >> 5, gstride >> 5, stage[threadIdx.x >> 5]);
                 if (!grid_barrier(a.bar)) return;
                 fx_finalize_range<M>(st, gtid, gstride);
                 if (!grid_barrier(a.bar)) return;
             } else {
-                apply_range<M>(st, item0, c, 0, a.cand_dest, a.cand_prio, gtid, gstride);
+                apply_range<M>(st, item0, cnt, c, 0, gtid >> 5, gstride >> 5);
                 if (!grid_barrier(a.bar)) return;
                 for (int r = 1; r < a.match_rounds; r++) {
-                    reclaim_range(st, item0, c, r, a.cand_dest, a.cand_prio, gtid, gstride);
+                    reclaim_range(st, item0, c, r, gtid, gstride);
                     if (!grid_barrier(a.bar)) return;
-                    apply_range<M>(st, item0, c, r, a.cand_dest, a.cand_prio, gtid, gstride);
+                    apply_range<M>(st, item0, cnt, c, r, gtid >> 5, gstride >> 5);
                     if (!grid_barrier(a.bar)) return;
                 }
             }
@@ -2082,15 +2205,13 @@ static int screen_blocks_per_sm(int metric) {
     return (e == cudaSuccess && nb > 0) ? nb : 1;
 }
 
-cudaError_t launch_eval(int metric, const DevState& st, int item0, int64_t count, int color,
-                        int* cand_dest, unsigned* cand_prio, bool claims, bool split, int blocks, int threads,
-                        cudaStream_t s) {
+cudaError_t launch_eval(int metric, const DevState& st, int item0, int64_t count, int color, bool claims, bool split,
+                        int blocks, int threads, cudaStream_t s) {
     if (count == 0) return cudaSuccess;
     if (threads == 128) {
         // 128-thread blocks, as many threads per SM as four blocks of 256
         if (!split) {
-            ACVD_DISPATCH_128(metric, eval_kernel, nblk(count, 128), s, st, item0, count, color, cand_dest,
-                              cand_prio, claims ? 1 : 0);
+            ACVD_DISPATCH_128(metric, eval_kernel, nblk(count, 128), s, st, item0, count, color, claims ? 1 : 0);
             return cudaGetLastError();
         }
         const unsigned sgrid =
@@ -2098,13 +2219,12 @@ cudaError_t launch_eval(int metric, const DevState& st, int item0, int64_t count
         ACVD_DISPATCH(metric, screen_kernel, sgrid, 256, s, st, item0, count, color, st.work, st.work_count);
         const int64_t tiles = kWorkStripes * (work_cap(count) / 128);
         const unsigned grid = (unsigned)std::min<int64_t>(tiles, sm_count() * eval_list_blocks_per_sm_128(metric));
-        ACVD_DISPATCH_128(metric, eval_list_kernel, grid, s, st, item0, count, color, cand_dest, cand_prio,
-                          claims ? 1 : 0, (const int*)st.work, (const unsigned*)st.work_count);
+        ACVD_DISPATCH_128(metric, eval_list_kernel, grid, s, st, item0, count, color, claims ? 1 : 0, (const int*)st.work, (const unsigned*)st.work_count);
         return cudaGetLastError();
     }
     if (!split) {
         ACVD_DISPATCH_B(metric, blocks, default_eval_blocks(metric), eval_kernel, nblk(count), 256, s, st, item0,
-                        count, color, cand_dest, cand_prio, claims ? 1 : 0);
+                        count, color, claims ? 1 : 0);
         return cudaGetLastError();
     }
     const unsigned sgrid = (unsigned)std::min<int64_t>(nblk(count, kScreenTile), sm_count() * screen_blocks_per_sm(metric));
@@ -2112,7 +2232,7 @@ cudaError_t launch_eval(int metric, const DevState& st, int item0, int64_t count
     const int64_t tiles = kWorkStripes * (work_cap(count) / 256);
     const unsigned grid = (unsigned)std::min<int64_t>(tiles, sm_count() * eval_list_blocks_per_sm(metric, blocks));
     ACVD_DISPATCH_B(metric, blocks, kDefaultListBlocks, eval_list_kernel, grid, 256, s, st, item0, count, color,
-                    cand_dest, cand_prio, claims ? 1 : 0, (const int*)st.work, (const unsigned*)st.work_count);
+                    claims ? 1 : 0, (const int*)st.work, (const unsigned*)st.work_count);
     return cudaGetLastError();
 }
 
@@ -2129,25 +2249,30 @@ static unsigned list_grid(int64_t count) {
     return (unsigned)std::min<int64_t>(nblk(count), 2 * sm_count());
 }
 
+// Blocks of the commit kernels: a warp for every 32 items of the class, at most 16 warps
+// to an SM (2,432 on a 152-SM GB300; more proposals than that take further lanes of them)
+static unsigned commit_grid(int64_t count) {
+    return (unsigned)std::min<int64_t>(nblk(count, kCommitThreads), 4 * sm_count());
+}
+
 cudaError_t launch_apply(int metric, const DevState& st, int item0, int64_t count, int color, int round,
-                         int* cand_dest, const unsigned* cand_prio, cudaStream_t s) {
+                         cudaStream_t s) {
     if (count == 0) return cudaSuccess;
-    ACVD_DISPATCH(metric, apply_kernel, list_grid(count), 256, s, st, item0, color, round, cand_dest, cand_prio);
+    ACVD_DISPATCH(metric, apply_kernel, commit_grid(count), kCommitThreads, s, st, item0, count, color, round);
     return cudaGetLastError();
 }
 
-cudaError_t launch_reclaim(const DevState& st, int item0, int64_t count, int color, int round,
-                           int* cand_dest, const unsigned* cand_prio, cudaStream_t s) {
+cudaError_t launch_reclaim(const DevState& st, int item0, int64_t count, int color, int round, cudaStream_t s) {
     if (count == 0) return cudaSuccess;
     ++g_launches;
-    reclaim_kernel<<<list_grid(count), 256, 0, s>>>(st, item0, color, round, cand_dest, cand_prio);
+    reclaim_kernel<<<list_grid(count), 256, 0, s>>>(st, item0, color, round);
     return cudaGetLastError();
 }
 
 cudaError_t launch_relaxed_step(int metric, const DevState& st, int item0, int64_t count, int color,
-                                const int* cand_dest, cudaStream_t s) {
+                                cudaStream_t s) {
     if (count == 0) return cudaSuccess;
-    ACVD_DISPATCH(metric, relaxed_commit_kernel, list_grid(count), 256, s, st, item0, color, cand_dest);
+    ACVD_DISPATCH(metric, relaxed_commit_kernel, commit_grid(count), kCommitThreads, s, st, item0, count, color);
     ACVD_DISPATCH(metric, fx_finalize_kernel, nblk(st.k, 64), 64, s, st);   // small blocks: every SM gets some
     return cudaGetLastError();
 }
@@ -2166,12 +2291,24 @@ cudaError_t launch_begin_sweep(const DevState& st, int ncolors, bool reset_claim
     return cudaGetLastError();
 }
 
+static const void* sweep_run_fn(int metric) {
+    return metric == kIso ? (const void*)sweep_run_kernel<kIso>
+         : metric == kQEM ? (const void*)sweep_run_kernel<kQEM>
+                          : (const void*)sweep_run_kernel<kAniso>;
+}
+
+static size_t sweep_run_stage_bytes(int metric) {
+    return 8 * (metric == kIso ? sizeof(CommitStage<kIso>)
+              : metric == kQEM ? sizeof(CommitStage<kQEM>) : sizeof(CommitStage<kAniso>));
+}
+
 int sweep_run_blocks_per_sm(int metric) {
     int nb = 0;
     cudaError_t e;
-    if (metric == kIso) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sweep_run_kernel<kIso>, 256, 0);
-    else if (metric == kQEM) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sweep_run_kernel<kQEM>, 256, 0);
-    else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sweep_run_kernel<kAniso>, 256, 0);
+    const int sm = (int)sweep_run_stage_bytes(metric);
+    const void* fn = sweep_run_fn(metric);
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 256, sm);
     return e == cudaSuccess ? nb : 0;
 }
 
@@ -2179,10 +2316,8 @@ cudaError_t launch_sweep_run(int metric, const SweepRun& a, int grid, cudaStream
     ++g_launches;
     SweepRun arg = a;
     void* args[] = {(void*)&arg};
-    const void* fn = metric == kIso ? (const void*)sweep_run_kernel<kIso>
-                     : metric == kQEM ? (const void*)sweep_run_kernel<kQEM>
-                                      : (const void*)sweep_run_kernel<kAniso>;
-    return cudaLaunchCooperativeKernel(fn, dim3((unsigned)grid), dim3(256), args, 0, s);
+    return cudaLaunchCooperativeKernel(sweep_run_fn(metric), dim3((unsigned)grid), dim3(256), args,
+                                       sweep_run_stage_bytes(metric), s);
 }
 
 cudaError_t launch_update_all(int metric, const DevState& st, cudaStream_t s) {

@@ -55,7 +55,8 @@ struct acvd_ctx {
     DBuf<unsigned> adj;
     int ncolors = 0;
     std::vector<int64_t> color_off;
-    DBuf<int> color_items, cand_dest, cand_list;
+    DBuf<int> color_items;
+    DBuf<int4> cand_list;
     // acvd_adjoint_on_stream: orders the context's stream after the caller's and back
     cudaEvent_t adj_ev_in = nullptr, adj_ev_out = nullptr;
     // split evaluation of large colour classes (screen pass + work list)
@@ -83,7 +84,7 @@ struct acvd_ctx {
     std::vector<int64_t> sweep_off;
     const int* sweep_items = nullptr;
     int nclasses = 0;
-    DBuf<unsigned> cand_prio, cand_count;
+    DBuf<unsigned> cand_count;
 
     // batch of meshes packed in one CSR (vertex and cluster offsets per mesh)
     int nmesh = 0;
@@ -516,12 +517,9 @@ static int setup_colors(acvd_ctx* ctx, const int32_t* h_row, const int32_t* h_co
         }
         ctx->has_work = wmax > 0;
     }
-    CK(ctx->cand_dest.resize(mx));
-    CK(ctx->cand_prio.resize(mx));
     CK(ctx->cand_list.resize(mx));
     CK(ctx->cand_count.resize(64));
     CK(ctx->evald.resize(n));
-    CK(cudaMemsetAsync(ctx->cand_dest.p, 0xff, mx * sizeof(int), ctx->s));
     CK(cudaMemsetAsync(ctx->cand_count.p, 0, 64 * sizeof(unsigned), ctx->s));
     return ACVD_OK;
 }
@@ -1087,20 +1085,19 @@ static int enqueue_sweep(acvd_ctx* ctx, bool timing, bool relaxed) {
         // cudaEventRecordExternal makes the records real graph nodes when captured
         if (timing) CK(cudaEventRecordWithFlags(ctx->ev_eval[2 * c], ctx->s, cudaEventRecordExternal));
         const bool split = ctx->has_work && ctx->split_min > 0 && cnt >= ctx->split_min;
-        CK(launch_eval(ctx->metric, st, item0, cnt, c, ctx->cand_dest.p, ctx->cand_prio.p, !relaxed, split,
-                       ctx->eval_blocks, ctx->eval_threads, ctx->s));
+        CK(launch_eval(ctx->metric, st, item0, cnt, c, !relaxed, split, ctx->eval_blocks, ctx->eval_threads, ctx->s));
         if (split) kernels++;
         if (timing) CK(cudaEventRecordWithFlags(ctx->ev_eval[2 * c + 1], ctx->s, cudaEventRecordExternal));
         if (relaxed) {
-            CK(launch_relaxed_step(ctx->metric, st, item0, cnt, c, ctx->cand_dest.p, ctx->s));
+            CK(launch_relaxed_step(ctx->metric, st, item0, cnt, c, ctx->s));
             kernels += 3;
             continue;
         }
-        CK(launch_apply(ctx->metric, st, item0, cnt, c, 0, ctx->cand_dest.p, ctx->cand_prio.p, ctx->s));
+        CK(launch_apply(ctx->metric, st, item0, cnt, c, 0, ctx->s));
         kernels += 2;
         for (int r = 1; r < ctx->match_rounds; r++) {
-            CK(launch_reclaim(st, item0, cnt, c, r, ctx->cand_dest.p, ctx->cand_prio.p, ctx->s));
-            CK(launch_apply(ctx->metric, st, item0, cnt, c, r, ctx->cand_dest.p, ctx->cand_prio.p, ctx->s));
+            CK(launch_reclaim(st, item0, cnt, c, r, ctx->s));
+            CK(launch_apply(ctx->metric, st, item0, cnt, c, r, ctx->s));
             kernels += 2;
         }
     }
@@ -1298,8 +1295,6 @@ static int run_sweeps_persistent(acvd_ctx* ctx, LoopState& hl, acvd_stats& local
     a.off = ctx->doff.p;
     a.nclasses = ctx->nclasses;
     a.match_rounds = ctx->match_rounds;
-    a.cand_dest = ctx->cand_dest.p;
-    a.cand_prio = ctx->cand_prio.p;
     a.ls = ctx->dls.p;
     a.bar = ctx->dbar.p;
     a.esum = ctx->esum.p;

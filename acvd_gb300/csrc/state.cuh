@@ -182,7 +182,8 @@ struct DevState {
     SweepState* sweep;     // sweep counter / invalidation floor
     int* stamp;            // per cluster: sweep of its last modification
     int* evald;            // per item: sweep of its last evaluation without a proposal (-1: none)
-    int* cand_list;        // compact list of proposals (colour-list positions) of the current step
+    int4* cand_list;       // compact list of the step's proposals: class position, destination cluster
+                           // (-1 once committed or dropped), source cluster, priority
     unsigned* cand_count;  // per colour: number of proposals
     // relaxed steps: per cluster, exact fixed-point sums of the committed moves'
     // contributions (order-independent, hence deterministic with atomics)
@@ -272,8 +273,6 @@ struct SweepRun {
     const long long* off;     // class offsets (nclasses + 1)
     int nclasses;
     int match_rounds;
-    int* cand_dest;
-    unsigned* cand_prio;
     LoopState* ls;
     GridBar* bar;
     double* esum;             // energy-sum partials: ceil(K/2048) + ceil(K/2048^2) + 2 doubles
@@ -335,18 +334,15 @@ cudaError_t launch_loop_start(const LoopState* ls, const RunFlags* flags, cudaGr
 cudaError_t launch_loop_decide(LoopState* ls, const unsigned long long* counters, const double* e_now,
                                const RunFlags* flags, bool relaxed, cudaGraphConditionalHandle h_loop,
                                cudaGraphConditionalHandle h_mode, cudaStream_t s);
-cudaError_t launch_relaxed_step(int metric, const DevState& st, int item0, int64_t count, int color,
-                                const int* cand_dest, cudaStream_t s);
+cudaError_t launch_relaxed_step(int metric, const DevState& st, int item0, int64_t count, int color, cudaStream_t s);
 cudaError_t launch_fx_scale(int metric, const DevState& st, unsigned* maxbits, cudaStream_t s);
 // blocks: 256-thread blocks per SM (3..5, else the defaults); threads: 128 for
 // 128-thread blocks at the threads per SM of four 256-thread blocks (else 256)
-cudaError_t launch_eval(int metric, const DevState& st, int item0, int64_t count, int color,
-                        int* cand_dest, unsigned* cand_prio, bool claims, bool split, int blocks, int threads,
-                        cudaStream_t s);
+cudaError_t launch_eval(int metric, const DevState& st, int item0, int64_t count, int color, bool claims, bool split,
+                        int blocks, int threads, cudaStream_t s);
 cudaError_t launch_apply(int metric, const DevState& st, int item0, int64_t count, int color, int round,
-                         int* cand_dest, const unsigned* cand_prio, cudaStream_t s);
-cudaError_t launch_reclaim(const DevState& st, int item0, int64_t count, int color, int round,
-                           int* cand_dest, const unsigned* cand_prio, cudaStream_t s);
+                         cudaStream_t s);
+cudaError_t launch_reclaim(const DevState& st, int item0, int64_t count, int color, int round, cudaStream_t s);
 // Persistent sweep kernel (cooperative launch).  blocks_per_sm: co-resident
 // blocks per SM for this metric (0 when the kernel cannot be co-resident).
 int sweep_run_blocks_per_sm(int metric);

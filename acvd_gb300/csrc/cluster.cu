@@ -24,6 +24,34 @@ namespace acvd {
 // relative margin an energy decrease must exceed to be proposed (about 100 float32 ulps)
 constexpr float kAcceptTol = 1e-5f;
 
+// A load issued here, not sunk to where its value is used (behind a branch that most of
+// the loads' latency would then follow).
+ACVD_DEV float2 load_now(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+ACVD_DEV float4 load_now(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+ACVD_DEV int4 load_now(const int4* p) {
+    int4 v;
+    asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+ACVD_DEV int load_now(const int* p) {
+    int v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+ACVD_DEV double load_now(const double* p) {
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
 struct ItemRec {
     float x[3];
     float w;
@@ -308,6 +336,8 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
     __shared__ unsigned char s_rem[TB];                // work items whose remove part B1 computes
     __shared__ int s_scr[TB];                 // flagged items of the tile (colour-list positions)
     __shared__ unsigned char s_rec[TB];       // work item -> its screen record is valid (bflag 2)
+    __shared__ int4 s_scn[TB];                // ... and that record (its evaluation sweep aside)
+    __shared__ int s_lab[TB];                 // work item -> its cluster
     __shared__ unsigned s_nwork, s_ntask, s_nrem, s_nscr, s_nfull;
     __syncthreads();                     // the previous tile is done with the shared arrays
     if (threadIdx.x == 0) {
@@ -353,12 +383,22 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
         const int64_t idx = code & ~kScrCached;
         const int i = item0 + (int)idx;
         n_scr = 1;
-        // a cached screen's record holds the item's cluster and evaluation sweep too
+        // a cached screen's record holds the item's cluster and evaluation sweep too; a full
+        // screen starts from the item's label, evaluation sweep and ring, loaded together
         const bool cached = (code & kScrCached) != 0;
-        const int4 c = cached ? st.tcache[i] : make_int4(0, 0, 0, 0);
+        int4 c = make_int4(0, 0, 0, 0), ra = c, rb = c;
+        int lab_i = 0, evald_i = 0;
+        if (cached) {
+            c = load_now(st.tcache + i);
+        } else {
+            lab_i = load_now(st.label + i);
+            evald_i = load_now(st.evald + i);
+            ra = load_now(st.ring8 + 2 * (int64_t)i);
+            rb = load_now(st.ring8 + 2 * (int64_t)i + 1);
+        }
         const Screen sc = unpack_screen(c);
-        const int L = cached ? sc.L : st.label[i];
-        int ev_i = cached ? sc.ev : st.evald[i];
+        const int L = cached ? sc.L : lab_i;
+        int ev_i = cached ? sc.ev : evald_i;
         if (cached) ACVD_VALID(st, L == st.label[i] && ev_i == st.evald[i]);
         bool screened = !ACVD_VALID(st, L >= 0 && L <= st.k);   // a bad label is skipped
         if (cached && !screened) {
@@ -366,21 +406,25 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
             // neighbour clusters and the connectivity test are in the cache
             const int n = sc.n;
             const bool conn_known = sc.conn_known, conn_ok = sc.conn_ok;
-            const bool may_move = st.size[L] > 1 && !(st.frozen && st.frozen[L]);
+            // the size and every stamp in one go (unused targets are cluster 0)
+            const int tg[3] = {sc.t[0], sc.t[1], sc.t[2]};
+            const int size = load_now(st.size + L), stamp = load_now(st.stamp + L);
+            const int st0 = load_now(st.stamp + tg[0]), st1 = load_now(st.stamp + tg[1]),
+                      st2 = load_now(st.stamp + tg[2]);
+            const bool may_move = size > 1 && !(st.frozen && st.frozen[L]);
             if (!(fl.connexity && may_move && !conn_known)) {
                 screened = true;
                 n_cached = 1;
-                const int tg[3] = {sc.t[0], sc.t[1], sc.t[2]};
-                bool fresh = ev_i <= sw.floor || st.stamp[L] >= ev_i;
-#pragma unroll
-                for (int q = 0; q < 3; q++)
-                    if (q < n && st.stamp[tg[q]] >= ev_i) fresh = true;
+                const bool fresh = ev_i <= sw.floor || stamp >= ev_i || (n > 0 && st0 >= ev_i) ||
+                                   (n > 1 && st1 >= ev_i) || (n > 2 && st2 >= ev_i);
                 if (fresh) {
                     n_bnd = 1;
                     if (may_move && (!fl.connexity || conn_ok)) {
                         const int w = (int)atomicAdd(&s_nwork, 1u);
                         s_idx[w] = (int)idx;
+                        s_lab[w] = L;
                         s_rec[w] = 1;
+                        s_scn[w] = c;
                         int nt = 0;
 #pragma unroll
                         for (int q = 0; q < 3; q++)
@@ -400,7 +444,10 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
             }
         }
         if (!screened) {
-        const int4 ra = st.ring8[2 * (int64_t)i], rb = st.ring8[2 * (int64_t)i + 1];
+        if (cached) {   // its connectivity test is not known yet: the full screen after all
+            ra = st.ring8[2 * (int64_t)i];
+            rb = st.ring8[2 * (int64_t)i + 1];
+        }
         int lb[kRingPref] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
         const bool longer = lb[7] == -2;   // ring longer than 8: bounds and tail from the CSR
         int deg = 0;
@@ -412,8 +459,13 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
             for (int q = 0; q < kRingPref; q++) deg += lb[q] >= 0;
         }
 #pragma unroll
-        for (int q = 0; q < kRingPref; q++) lb[q] = lb[q] >= 0 ? st.label[lb[q]] : L;
-        bool fresh = ev_i <= sw.floor || (L < st.k && st.stamp[L] >= ev_i);
+        for (int q = 0; q < kRingPref; q++) lb[q] = lb[q] >= 0 ? load_now(st.label + lb[q]) : L;
+        // every stamp in one go (stamp[k], the null label's, exists and is not used)
+        int sb[kRingPref];
+        const int stamp = load_now(st.stamp + L), size = load_now(st.size + L);
+#pragma unroll
+        for (int q = 0; q < kRingPref; q++) sb[q] = lb[q] != L ? load_now(st.stamp + lb[q]) : 0;
+        bool fresh = ev_i <= sw.floor || (L < st.k && stamp >= ev_i);
         n_slots = (unsigned)deg;
         bool boundary = false;
 #pragma unroll
@@ -421,7 +473,7 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
             const int B = lb[q];
             if (B != L) {
                 boundary = true;
-                if (B < st.k && st.stamp[B] >= ev_i) fresh = true;
+                if (B < st.k && sb[q] >= ev_i) fresh = true;
             }
         }
         if (longer) {
@@ -435,7 +487,7 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
             }
         }
         if (!boundary) st.bflag[i] = 0;   // interior until a commit touches its ring
-        const bool may_move = L < st.k && st.size[L] > 1 && !(st.frozen && st.frozen[L]);
+        const bool may_move = L < st.k && size > 1 && !(st.frozen && st.frozen[L]);
         int conn = -1;   // the local connectivity test, evaluated at most once
         // cache a boundary screen of a ring of at most 8 with at most 3 neighbour
         // clusters: they hold until a commit touches the ring (mark_ring).  The record
@@ -474,7 +526,9 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
             if (movable) {
                 const int w = (int)atomicAdd(&s_nwork, 1u);
                 s_idx[w] = (int)idx;
+                s_lab[w] = L;
                 s_rec[w] = cache_it ? 1 : 0;
+                s_scn[w] = rec;
                 int nt = 0;
                 bool all = L < st.k && deg <= kRingPref;
 #pragma unroll
@@ -529,7 +583,7 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
         load_item<M>(st, i, it);
         if (j == kTaskRemove) {
             EvalRec eL;
-            load_eval<M>(st, st.label[i], eL);
+            load_eval<M>(st, s_lab[w], eL);
             float xc[3];
             s_val[w][kMaxTgt] = is_anchor_item<M>(eL, i) ? kBrokenAnchor : remove_part<M>(eL, it, fl, xc);
         } else {
@@ -545,7 +599,7 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
         const int w = threadIdx.x;
         const int widx = s_idx[w];
         const int i = item0 + widx;
-        const int L = st.label[i];
+        const int L = s_lab[w];
         const int nt = s_nt[w];
         int best = -1;
         unsigned pr = 0u;
@@ -615,10 +669,10 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
             n_cand = 1;
             my_cand = make_int4(widx, best, L, (int)pr);
             st.evald[i] = -1;
-            if (s_rec[w]) set_cached_ev(st, i, st.tcache[i], -1);
+            if (s_rec[w]) set_cached_ev(st, i, s_scn[w], -1);
         } else {
             st.evald[i] = sw.sweep;
-            if (s_rec[w]) set_cached_ev(st, i, st.tcache[i], sw.sweep);
+            if (s_rec[w]) set_cached_ev(st, i, s_scn[w], sw.sweep);
         }
     }
     // block-aggregated append to the compact proposal list and block totals of the
@@ -743,13 +797,22 @@ __global__ void __launch_bounds__(256, 4) screen_kernel(DevState st, int item0, 
         const int nc = (int)s_nc;
         for (int j0 = 0; j0 < nc; j0 += 256 * kScreenBatch) {
             // one 16-byte record per cached screen: cluster, targets, evaluation sweep
-            int pos[kScreenBatch];
+            int pos[kScreenBatch], size[kScreenBatch], stamp[kScreenBatch][4];
             int4 c[kScreenBatch];
 #pragma unroll
             for (int u = 0; u < kScreenBatch; u++) {
                 const int j = j0 + u * 256 + (int)threadIdx.x;
                 pos[u] = j < nc ? s_cached[j] : -1;
                 c[u] = pos[u] >= 0 ? st.tcache[item0 + (int)(t0 + pos[u])] : make_int4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < kScreenBatch; u++) {
+                const Screen sc = unpack_screen(c[u]);
+                const bool known = pos[u] >= 0 && sc.L <= st.k;
+                size[u] = known ? load_now(st.size + sc.L) : 0;
+                stamp[u][0] = known ? load_now(st.stamp + sc.L) : 0;
+#pragma unroll
+                for (int q = 0; q < 3; q++) stamp[u][q + 1] = known ? load_now(st.stamp + sc.t[q]) : 0;
             }
 #pragma unroll
             for (int u = 0; u < kScreenBatch; u++) {
@@ -761,13 +824,13 @@ __global__ void __launch_bounds__(256, 4) screen_kernel(DevState st, int item0, 
                 }
                 if (pos[u] < 0 || !ACVD_VALID(st, L >= 0 && L <= st.k)) continue;
                 const int n = sc.n;
-                const bool may_move = st.size[L] > 1 && !(st.frozen && st.frozen[L]);
+                const bool may_move = size[u] > 1 && !(st.frozen && st.frozen[L]);
                 bool fwd = fl.connexity && may_move && !sc.conn_known;   // connectivity not cached: full screen
                 if (!fwd) {
-                    bool fresh = ev_i <= sw.floor || st.stamp[L] >= ev_i;
+                    bool fresh = ev_i <= sw.floor || stamp[u][0] >= ev_i;
 #pragma unroll
                     for (int q = 0; q < 3; q++)
-                        if (q < n && st.stamp[sc.t[q]] >= ev_i) fresh = true;
+                        if (q < n && stamp[u][q + 1] >= ev_i) fresh = true;
                     if (fresh && may_move && (!fl.connexity || sc.conn_ok)) {
                         fwd = true;   // an energy test to run
                     } else {
@@ -1036,34 +1099,6 @@ ACVD_DEV void update_cluster(const DevState& st, int k) {
 // ---------------------------------------------------------------------------
 constexpr int kCommitThreads = 128;
 constexpr int kCommitWarps = kCommitThreads / 32;
-
-// A load issued here, not sunk to where its value is used (behind a branch that most of
-// the loads' latency would then follow).
-ACVD_DEV float2 load_now(const float2* p) {
-    float2 v;
-    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
-    return v;
-}
-ACVD_DEV float4 load_now(const float4* p) {
-    float4 v;
-    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-    return v;
-}
-ACVD_DEV int4 load_now(const int4* p) {
-    int4 v;
-    asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-ACVD_DEV int load_now(const int* p) {
-    int v;
-    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
-ACVD_DEV double load_now(const double* p) {
-    double v;
-    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
 
 template <int M>
 ACVD_DEV void load_item_now(const DevState& st, int i, ItemRec& it) {

@@ -66,15 +66,15 @@ __global__ void adj_clamp(AdjState a, const double* wsum, double ratio) {
 }
 
 // one warp per cluster over its items (sorted by cluster): FP64 sums, fixed order
-__global__ void adj_cluster_sums(AdjState a, const uint32_t* __restrict__ sorted, const uint32_t* __restrict__ off,
-                                 const uint32_t* __restrict__ cnt) {
+__global__ void adj_cluster_sums(AdjState a, const uint32_t* __restrict__ sorted, const uint32_t* __restrict__ off) {
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= a.k) return;
     double s[13];
     for (int q = 0; q < 13; q++) s[q] = 0.0;
-    for (uint32_t j = lane; j < cnt[w]; j += 32) {
-        const uint32_t i = sorted[off[w] + j];
+    const uint32_t s0 = off[w], s1 = off[w + 1];
+    for (uint32_t j = s0 + lane; j < s1; j += 32) {
+        const uint32_t i = sorted[j];
         const double wi = a.vw[i];
         const double xi[3] = {a.x[3 * i], a.x[3 * i + 1], a.x[3 * i + 2]};
         const double* Ai = a.vA + 6 * (int64_t)i;
@@ -291,14 +291,14 @@ static inline unsigned nb(int64_t n, int b = 256) { return (unsigned)((n + b - 1
 
 cudaError_t adjoint_run(const AdjState& a, int metric, int level, double thr, double ratio, double gE,
                         const double* dgE, const double* gC, const uint32_t* sorted, const uint32_t* off,
-                        const uint32_t* cnt, double* wsum, double* cent, double* gx, double* grho, cudaStream_t s,
+                        double* wsum, double* cent, double* gx, double* grho, cudaStream_t s,
                         Scratch& scratch) {
     adj_face_fwd<<<nb(a.nf), 256, 0, s>>>(a);
     adj_vertex_fwd<<<nb(a.nv), 256, 0, s>>>(a);
     cudaError_t e = sum_f64(a.vw, a.nv, wsum, scratch, s);
     if (e != cudaSuccess) return e;
     adj_clamp<<<nb(a.nv), 256, 0, s>>>(a, wsum, ratio);
-    adj_cluster_sums<<<nb((int64_t)a.k * 32), 256, 0, s>>>(a, sorted, off, cnt);
+    adj_cluster_sums<<<nb((int64_t)a.k * 32), 256, 0, s>>>(a, sorted, off);
     adj_cluster<<<nb(a.k, 128), 128, 0, s>>>(a, metric, level, thr, gE, dgE, gC, cent);
     g_launches += 6;
     if (gx) {

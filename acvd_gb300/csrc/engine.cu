@@ -947,22 +947,28 @@ int acvd_rewind(acvd_ctx* ctx) {
 // ---------------------------------------------------------------------------
 // MinimizeEnergy building blocks
 // ---------------------------------------------------------------------------
-static int recompute(acvd_ctx* ctx) {
-    DevState st = ctx->state();
+// The items by cluster: wk_b holds them sorted (the unassigned ones last), cluster c's at
+// wk_off[c] .. wk_off[c + 1].  st.label may be in item order or in vertex order.
+static int group_by_cluster(acvd_ctx* ctx, const DevState& st) {
     const int64_t n = ctx->nV;
     const int K = ctx->K;
     CK(ctx->wk_a.resize(n));
     CK(ctx->wk_b.resize(n));
     CK(ctx->wk_c.resize(n));
     CK(ctx->wk_d.resize(n));
-    CK(ctx->wk_cnt.resize(K + 1));
-    CK(ctx->wk_off.resize(K + 1));
-    CK(cudaMemsetAsync(ctx->wk_cnt.p, 0, (K + 1) * sizeof(uint32_t), ctx->s));
-    CK(launch_cluster_keys(st, ctx->wk_a.p, ctx->wk_b.p, ctx->wk_cnt.p, ctx->s));
+    CK(ctx->wk_off.resize(K + 2));
+    CK(launch_cluster_keys(st, ctx->wk_a.p, ctx->wk_b.p, ctx->s));
     CK(radix_sort_pairs(ctx->wk_a.p, ctx->wk_b.p, ctx->wk_c.p, ctx->wk_d.p, n, bits_for((uint64_t)K), ctx->scratch,
                         ctx->s));
-    CK(exclusive_scan_u32(ctx->wk_cnt.p, ctx->wk_off.p, K + 1, nullptr, ctx->scratch, ctx->s));
-    CK(launch_reduce_clusters(ctx->metric, st, ctx->wk_b.p, ctx->wk_off.p, ctx->wk_cnt.p, ctx->s));
+    CK(launch_segment_offsets(ctx->wk_a.p, n, (uint32_t)K + 1u, ctx->wk_off.p, ctx->s));
+    return ACVD_OK;
+}
+
+static int recompute(acvd_ctx* ctx) {
+    DevState st = ctx->state();
+    const int r = group_by_cluster(ctx, st);
+    if (r) return r;
+    CK(launch_reduce_clusters(ctx->metric, st, ctx->wk_b.p, ctx->wk_off.p, ctx->s));
     CK(launch_update_all(ctx->metric, st, ctx->s));
     return ACVD_OK;
 }
@@ -1886,19 +1892,12 @@ extern "C" int acvd_post_placement(acvd_ctx* ctx, int level, double* points) {
     CK(launch_gather_i32(ctx->label.p, ctx->inv.p, nv, ctx->label_orig.p, ctx->s));
     DevState st = ctx->state();
     st.label = ctx->label_orig.p;
-    CK(ctx->wk_a.resize(nv)); CK(ctx->wk_b.resize(nv)); CK(ctx->wk_c.resize(nv)); CK(ctx->wk_d.resize(nv));
-    CK(ctx->wk_cnt.resize(K + 1)); CK(ctx->wk_off.resize(K + 1));
-    CK(cudaMemsetAsync(ctx->wk_cnt.p, 0, (K + 1) * sizeof(uint32_t), ctx->s));
-    CK(launch_cluster_keys(st, ctx->wk_a.p, ctx->wk_b.p, ctx->wk_cnt.p, ctx->s));
-    CK(radix_sort_pairs(ctx->wk_a.p, ctx->wk_b.p, ctx->wk_c.p, ctx->wk_d.p, nv, bits_for((uint64_t)K), ctx->scratch,
-                        ctx->s));
-    CK(exclusive_scan_u32(ctx->wk_cnt.p, ctx->wk_off.p, K + 1, nullptr, ctx->scratch, ctx->s));
+    if ((r = group_by_cluster(ctx, st))) return r;
     CK(qv.resize(9 * (size_t)nv));
     CK(launch_vertex_quadrics(ctx->xyz.p, ctx->tri.p, ctx->vf_row.p, ctx->vf_face.p, nv, qv.p, ctx->s));
     CK(out.resize(3 * (size_t)K));
     CK(ctx->dtmp.resize(2));
-    CK(launch_post_place(qv.p, ctx->wk_b.p, ctx->wk_off.p, ctx->wk_cnt.p, (const int*)ctx->wk_cnt.p, (int*)ctx->dtmp.p,
-                         start.p, K, level, out.p, ctx->s));
+    CK(launch_post_place(qv.p, ctx->wk_b.p, ctx->wk_off.p, (int*)ctx->dtmp.p, start.p, K, level, out.p, ctx->s));
     CK(cudaMemcpyAsync(points, out.p, 3 * (size_t)K * sizeof(double), cudaMemcpyDeviceToHost, ctx->s));
     CK(cudaStreamSynchronize(ctx->s));
     return ACVD_OK;
@@ -2244,7 +2243,7 @@ extern "C" int acvd_get_dual_mesh(acvd_ctx* ctx, int32_t* tris, int64_t* n_tris)
 namespace acvd {
 cudaError_t adjoint_run(const AdjState& a, int metric, int level, double thr, double ratio, double gE,
                         const double* dgE, const double* gC, const uint32_t* sorted, const uint32_t* off,
-                        const uint32_t* cnt, double* wsum, double* cent, double* gx, double* grho, cudaStream_t s,
+                        double* wsum, double* cent, double* gx, double* grho, cudaStream_t s,
                         Scratch& scratch);
 }  // namespace acvd
 
@@ -2262,13 +2261,10 @@ static int adjoint_enqueue(acvd_ctx* ctx, const double* xyz, const double* rho, 
     CK(launch_gather_i32(ctx->label.p, ctx->inv.p, nv, ctx->label_orig.p, ctx->s));
     DevState st = ctx->state();
     st.label = ctx->label_orig.p;
-    CK(ctx->wk_a.resize(nv)); CK(ctx->wk_b.resize(nv)); CK(ctx->wk_c.resize(nv)); CK(ctx->wk_d.resize(nv));
-    CK(ctx->wk_cnt.resize(K + 1)); CK(ctx->wk_off.resize(K + 1));
-    CK(cudaMemsetAsync(ctx->wk_cnt.p, 0, (K + 1) * sizeof(uint32_t), ctx->s));
-    CK(launch_cluster_keys(st, ctx->wk_a.p, ctx->wk_b.p, ctx->wk_cnt.p, ctx->s));
-    CK(radix_sort_pairs(ctx->wk_a.p, ctx->wk_b.p, ctx->wk_c.p, ctx->wk_d.p, nv, bits_for((uint64_t)K), ctx->scratch,
-                        ctx->s));
-    CK(exclusive_scan_u32(ctx->wk_cnt.p, ctx->wk_off.p, K + 1, nullptr, ctx->scratch, ctx->s));
+    {
+        const int r = group_by_cluster(ctx, st);
+        if (r) return r;
+    }
     CK(ctx->adj_work.resize(adjoint_bytes(nv, nf, K) + 64));
     AdjState a = adjoint_state(ctx->adj_work.p, nv, nf, K);
     a.x = xyz;
@@ -2281,7 +2277,7 @@ static int adjoint_enqueue(acvd_ctx* ctx, const double* xyz, const double* rho, 
     CK(ctx->dtmp.resize(4));
     const double ratio = ctx->metric == kQEM ? 10000.0 : 100000.0;
     CK(adjoint_run(a, ctx->metric, ctx->level, 1e-3, ratio, g_energy, d_g_energy, g_centroids, ctx->wk_b.p,
-                   ctx->wk_off.p, ctx->wk_cnt.p, ctx->dtmp.p, centroids, grad_xyz, grad_rho, ctx->s, ctx->scratch));
+                   ctx->wk_off.p, ctx->dtmp.p, centroids, grad_xyz, grad_rho, ctx->s, ctx->scratch));
     if (energy || d_energy) {
         CK(sum_f64(a.ek, K, ctx->dtmp.p + 1, ctx->scratch, ctx->s));
         if (d_energy) CK(cudaMemcpyAsync(d_energy, ctx->dtmp.p + 1, sizeof(double), cudaMemcpyDeviceToDevice, ctx->s));

@@ -348,10 +348,10 @@ cudaError_t launch_reclaim(const DevState& st, int item0, int64_t count, int col
 int sweep_run_blocks_per_sm(int metric);
 cudaError_t launch_sweep_run(int metric, const SweepRun& a, int grid, cudaStream_t s);
 cudaError_t launch_update_all(int metric, const DevState& st, cudaStream_t s);
-cudaError_t launch_cluster_keys(const DevState& st, uint32_t* keys, uint32_t* vals, uint32_t* counts,
-                                cudaStream_t s);
+cudaError_t launch_cluster_keys(const DevState& st, uint32_t* keys, uint32_t* vals, cudaStream_t s);
+// cluster c's items at sorted_items[seg_off[c] .. seg_off[c + 1])
 cudaError_t launch_reduce_clusters(int metric, const DevState& st, const uint32_t* sorted_items,
-                                   const uint32_t* seg_off, const uint32_t* seg_cnt, cudaStream_t s);
+                                   const uint32_t* seg_off, cudaStream_t s);
 cudaError_t launch_comp_init(const DevState& st, int* comp, cudaStream_t s);
 cudaError_t launch_comp_step(const DevState& st, int* comp, cudaStream_t s);
 // the components in one union-find pass, at most `tries` attempts per link; kCntChanged
@@ -384,9 +384,8 @@ cudaError_t launch_dual_write(const int* tri, const int* faces, const int* sel, 
 cudaError_t launch_centroids(int metric, const DevState& st, double* out, cudaStream_t s);
 cudaError_t launch_vertex_quadrics(const double* xyz, const int* tri, const uint32_t* vf_row, const uint32_t* vf_face,
                                    int64_t nv, double* qv, cudaStream_t s);
-cudaError_t launch_post_place(const double* qv, const uint32_t* sorted, const uint32_t* seg_off,
-                              const uint32_t* seg_cnt, const int* size, int* first, const double* start, int k,
-                              int level, double* out, cudaStream_t s);
+cudaError_t launch_post_place(const double* qv, const uint32_t* sorted, const uint32_t* seg_off, int* first,
+                              const double* start, int k, int level, double* out, cudaStream_t s);
 
 // ---- curvature (curvature.cu) ----
 size_t curvature_face_bytes(int64_t nf);

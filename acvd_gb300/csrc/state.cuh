@@ -433,6 +433,8 @@ cudaError_t launch_boundary_gather(const int* ids, int64_t nb, const int* edge_v
 
 // ---- adjoint (adjoint.cu) ----
 // Work arrays and inputs of the fixed-clustering adjoint (FP64).
+constexpr int kAdjSums = 14;   // doubles per cluster, even: records stay 16-byte aligned
+constexpr int kAdjCot = 14;
 struct AdjState {
     int64_t nv, nf;
     int k;
@@ -443,15 +445,16 @@ struct AdjState {
     const int* label;
     const uint32_t* vf_row;
     const uint32_t* vf_face;
-    double* fn;           // 3 nf unit normals
-    double* flen;         // nf |cr|
-    double* farea;        // nf
-    double* va;           // nv dual areas
+    double* face;         // 4 nf: unit normal, |cr|
+    double* edge;         // 6 nf: gradients of the face's edge vectors p1 - p0, p2 - p0
     double* vA;           // 6 nv quadrics
-    double* vw;           // nv weights (clamped)
-    unsigned char* vclamp;
-    double* cl;           // per cluster: S(3) W A(6) b(3) | E | c(3) | GS(3) GW GA(6) Gb(3)
-    double* corner;       // 9 nf corner gradients
+    double* va;           // nv dual areas
+    double* vw;           // nv weights, not clamped
+    double* vrg;          // nv rho^g (with rho)
+    double* vga;          // nv dL/d(dual area) / 3, 0 where the weight is clamped
+    double* cl;           // per cluster kAdjSums: S(3) W A(6) b(3)
+    double* ct;           // per cluster kAdjCot: GS(3) GW GA(6) Gb(3), the cotangents of the sums
+    double* lim;          // 2: lower and upper clamp of the weights
     double* ek;           // k per-cluster energies
 };
 

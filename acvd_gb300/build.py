@@ -23,7 +23,7 @@ LIB_PLAIN = os.path.join(OUT, "libacvd_gb300_plain.so")
 PLAIN_SOURCE = "cluster.cu"
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 CU_SOURCES = ["primitives.cu", "topology.cu", "cluster.cu", "adjoint.cu", "engine.cu", "noalloc.cu", "curvature.cu", "subdivide.cu",
-              "manifold.cu"]
+              "manifold.cu", "dual.cu"]
 # per-file flags: the curvature kernel keeps every FP64 product and sum separately
 # rounded, so that it reproduces the CPU restatement bit for bit
 CU_FILE_FLAGS = {"curvature.cu": ["-fmad=false"]}

@@ -1008,9 +1008,10 @@ ACVD_DEV double cluster_record_df(const df* a, const RunFlags& fl, float4* ev, c
 
 // Record and energy of cluster k.  FULL: the quadric placement with the
 // reference's thresholded pseudo-inverse in FP64 (full recompute, final
-// results).  Otherwise the double-float path above.
+// results), the placed vertex in cent[0 .. 2] when that is given (an output vertex of the
+// coarse mesh).  Otherwise the double-float path above.
 template <int M, bool FULL>
-ACVD_DEV void update_cluster(const DevState& st, int k) {
+ACVD_DEV void update_cluster(const DevState& st, int k, double* cent = nullptr) {
     const df* a = st.acc + (int64_t)k * Layout<M>::acc;
     float4* ev = st.ev + (int64_t)k * Layout<M>::ev;
     if (!FULL) {
@@ -1032,9 +1033,12 @@ ACVD_DEV void update_cluster(const DevState& st, int k) {
         ev[0] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (M != kIso) for (int j = 1; j < Layout<M>::ev; j++) ev[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         st.energy[k] = 0.0;
+        const int ak = anchor_of<M>(st, k);
+        for (int j = 0; cent && j < 3; j++) cent[j] = ak >= 0 ? st.anchor_xyz[3 * (int64_t)k + j] : S[j] / W;
         return;
     }
     const double m[3] = {S[0] / W, S[1] / W, S[2] / W};
+    if (cent) { cent[0] = m[0]; cent[1] = m[1]; cent[2] = m[2]; }
     ev[0] = make_float4((float)m[0], (float)m[1], (float)m[2], (float)W);
     const double S2W = (S[0] * S[0] + S[1] * S[1] + S[2] * S[2]) / W;
     if (M == kIso) {
@@ -1056,6 +1060,7 @@ ACVD_DEV void update_cluster(const DevState& st, int k) {
         ev[3] = make_float4((float)A[0], (float)A[1], (float)A[2], (float)A[3]);
         ev[4] = make_float4((float)A[4], (float)A[5], 1.0f, __int_as_float(ak));
         st.energy[k] = (c[0] * c[0] + c[1] * c[1] + c[2] * c[2]) * W - 2.0 * (c[0] * S[0] + c[1] * S[1] + c[2] * S[2]);
+        if (cent) { cent[0] = c[0]; cent[1] = c[1]; cent[2] = c[2]; }
         return;
     }
     double Am[3];
@@ -1064,6 +1069,7 @@ ACVD_DEV void update_cluster(const DevState& st, int k) {
     double d[3] = {0.0, 0.0, 0.0};
     const bool place = (M == kAniso) || (fl.constrained && fl.level > 0);
     if (place) pinv_apply<double>(A, r, d, fl.level, (double)fl.thr, 32);
+    if (cent) { cent[0] = m[0] + d[0]; cent[1] = m[1] + d[1]; cent[2] = m[2] + d[2]; }
     const double P = W * (d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
     ev[1] = make_float4((float)d[0], (float)d[1], (float)d[2], (float)P);
     ev[2] = make_float4((float)r[0], (float)r[1], (float)r[2], 0.f);
@@ -1779,10 +1785,35 @@ __global__ void __launch_bounds__(256) reduce_clusters_kernel(DevState st, const
     if (lane == 0) st.size[w] = (int)cnt;
 }
 
+// The FP64 decompositions of the quadric metrics bound it (2 FP64 lanes per SM and cycle):
+// one warp per block, so that the SMs differ by one warp at most (20,000 clusters in 157
+// blocks of 128 put a second block on 5 of 152 SMs and took 63 us; 46 us so).  What
+// acvd_get_clusters returns is written along: the placed vertex needs no second
+// decomposition.
+constexpr int kUpdateThreads = 32;
+
 template <int M>
-__global__ void update_all_kernel(DevState st) {
-    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < st.k) update_cluster<M, true>(st, (int)k);
+__global__ void __launch_bounds__(kUpdateThreads) update_all_kernel(DevState st, ClusterOut out) {
+    const int64_t k = (int64_t)blockIdx.x * kUpdateThreads + threadIdx.x;
+    if (k >= st.k) return;
+    double c[3];
+    update_cluster<M, true>(st, (int)k, out.centroid ? c : nullptr);
+    const df* a = st.acc + k * Layout<M>::acc;
+    if (out.centroid)
+        for (int j = 0; j < 3; j++) out.centroid[3 * k + j] = c[j];
+    if (out.S)
+        for (int j = 0; j < 3; j++) out.S[3 * k + j] = df_to_d(a[j]);
+    if (out.W) out.W[k] = df_to_d(a[3]);
+    if (out.Q) {
+        // the reference's compact quadric: A entries and -b in slots 3, 6, 8
+        double q[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        if (M != kIso) {
+            q[0] = df_to_d(a[4]); q[1] = df_to_d(a[5]); q[2] = df_to_d(a[6]); q[3] = -df_to_d(a[10]);
+            q[4] = df_to_d(a[7]); q[5] = df_to_d(a[8]); q[6] = -df_to_d(a[11]); q[7] = df_to_d(a[9]);
+            q[8] = -df_to_d(a[12]);
+        }
+        for (int j = 0; j < 9; j++) out.Q[9 * k + j] = q[j];
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2003,99 +2034,10 @@ __global__ void __launch_bounds__(1024) fill_block_kernel(DevState st, const int
     warp_count(ctr(st.counters, kCntAssigned), done);
 }
 
-// ---------------------------------------------------------------------------
-// boundary edges, compaction, dual mesh
-// ---------------------------------------------------------------------------
-__global__ void boundary_edges_kernel(const int* __restrict__ ev, int64_t ne, const int* __restrict__ label,
-                                      uint32_t* __restrict__ flags) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= ne) return;
-    flags[e] = label[ev[2 * e]] != label[ev[2 * e + 1]] ? 1u : 0u;
-}
-
 __global__ void compact_kernel(const uint32_t* __restrict__ flags, const uint32_t* __restrict__ pos, int64_t n,
                                int* __restrict__ out) {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j < n && flags[j]) out[pos[j]] = (int)j;
-}
-
-__global__ void dual_faces_kernel(const int* __restrict__ tri, int64_t nf, const int* __restrict__ label, int k,
-                                  uint32_t* __restrict__ flags) {
-    const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nf) return;
-    const int a = label[tri[3 * f]], b = label[tri[3 * f + 1]], c = label[tri[3 * f + 2]];
-    flags[f] = (a < k && b < k && c < k && a >= 0 && b >= 0 && c >= 0 && a != b && b != c && a != c) ? 1u : 0u;
-}
-
-// canonical key of the sorted label triple s0 < s1 < s2 (21 bits each), split in
-// a low and a high 32-bit word
-__global__ void dual_keys_kernel(const int* __restrict__ tri, const int* __restrict__ faces, int64_t m,
-                                 const int* __restrict__ label, uint32_t* __restrict__ klo,
-                                 uint32_t* __restrict__ khi, uint32_t* __restrict__ order) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= m) return;
-    const int f = faces[j];
-    int a = label[tri[3 * f]], b = label[tri[3 * f + 1]], c = label[tri[3 * f + 2]];
-    if (a > b) { const int t = a; a = b; b = t; }
-    if (b > c) { const int t = b; b = c; c = t; }
-    if (a > b) { const int t = a; a = b; b = t; }
-    const unsigned long long key = ((unsigned long long)a << 42) | ((unsigned long long)b << 21) | (unsigned long long)c;
-    klo[j] = (uint32_t)(key & 0xffffffffull);
-    khi[j] = (uint32_t)(key >> 32);
-    order[j] = (uint32_t)j;
-}
-
-__global__ void gather_u32_kernel(const uint32_t* __restrict__ src, const uint32_t* __restrict__ idx, int64_t m,
-                                  uint32_t* __restrict__ dst) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < m) dst[j] = src[idx[j]];
-}
-
-// after the stable sort by (khi, klo): keep the first face of every distinct triple
-__global__ void dual_unique_kernel(const uint32_t* __restrict__ klo_sorted, const uint32_t* __restrict__ khi_sorted,
-                                   const uint32_t* __restrict__ order, int64_t m, uint32_t* __restrict__ keep) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= m) return;
-    const bool first = (j == 0) || klo_sorted[j] != klo_sorted[j - 1] || khi_sorted[j] != khi_sorted[j - 1];
-    keep[order[j]] = first ? 1u : 0u;
-}
-
-__global__ void dual_write_kernel(const int* __restrict__ tri, const int* __restrict__ faces,
-                                  const int* __restrict__ sel, int64_t t, const int* __restrict__ label,
-                                  int* __restrict__ out) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= t) return;
-    const int f = faces[sel[j]];
-    out[3 * j] = label[tri[3 * f]];
-    out[3 * j + 1] = label[tri[3 * f + 1]];
-    out[3 * j + 2] = label[tri[3 * f + 2]];
-}
-
-// FP64 placed vertex of every cluster (output vertices of the coarse mesh)
-template <int M>
-__global__ void centroids_kernel(DevState st, double* __restrict__ out) {
-    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= st.k) return;
-    if (anchor_of<M>(st, k) >= 0) {   // an anchored cluster's vertex is its anchor
-        for (int j = 0; j < 3; j++) out[3 * k + j] = st.anchor_xyz[3 * k + j];
-        return;
-    }
-    const df* a = st.acc + k * Layout<M>::acc;
-    const double W = df_to_d(a[3]);
-    double m[3] = {df_to_d(a[0]) / W, df_to_d(a[1]) / W, df_to_d(a[2]) / W};
-    if (M != kIso) {
-        const RunFlags fl = *st.flags;
-        if (M == kAniso || (fl.constrained && fl.level > 0)) {
-            double A[6], b[3], Am[3], d[3];
-            for (int j = 0; j < 6; j++) A[j] = df_to_d(a[4 + j]);
-            for (int j = 0; j < 3; j++) b[j] = df_to_d(a[10 + j]);
-            sym_mul<double>(A, m, Am);
-            const double r[3] = {b[0] - Am[0], b[1] - Am[1], b[2] - Am[2]};
-            pinv_apply<double>(A, r, d, fl.level, (double)fl.thr, 32);
-            m[0] += d[0]; m[1] += d[1]; m[2] += d[2];
-        }
-    }
-    out[3 * k] = m[0]; out[3 * k + 1] = m[1]; out[3 * k + 2] = m[2];
 }
 
 // ---------------------------------------------------------------------------
@@ -2365,9 +2307,9 @@ cudaError_t launch_sweep_run(int metric, const SweepRun& a, int grid, cudaStream
                                        sweep_run_stage_bytes(metric), s);
 }
 
-cudaError_t launch_update_all(int metric, const DevState& st, cudaStream_t s) {
+cudaError_t launch_update_all(int metric, const DevState& st, const ClusterOut& out, cudaStream_t s) {
     if (st.k == 0) return cudaSuccess;
-    ACVD_DISPATCH(metric, update_all_kernel, nblk(st.k, 128), 128, s, st);
+    ACVD_DISPATCH(metric, update_all_kernel, nblk(st.k, kUpdateThreads), kUpdateThreads, s, st, out);
     return cudaGetLastError();
 }
 
@@ -2439,63 +2381,10 @@ cudaError_t launch_fill_block(const DevState& st, const int* list, const int64_t
     return cudaGetLastError();
 }
 
-cudaError_t launch_boundary_edges(const int* edge_v, int64_t ne, const int* label, uint32_t* flags,
-                                  cudaStream_t s) {
-    if (ne == 0) return cudaSuccess;
-    ++g_launches;
-    boundary_edges_kernel<<<nblk(ne), 256, 0, s>>>(edge_v, ne, label, flags);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_compact(const uint32_t* flags, const uint32_t* pos, int64_t n, int* out, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     ++g_launches;
     compact_kernel<<<nblk(n), 256, 0, s>>>(flags, pos, n, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_dual_faces(const int* tri, int64_t nf, const int* label, int k, uint32_t* flags,
-                              cudaStream_t s) {
-    if (nf == 0) return cudaSuccess;
-    ++g_launches;
-    dual_faces_kernel<<<nblk(nf), 256, 0, s>>>(tri, nf, label, k, flags);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_dual_keys(const int* tri, const int* faces, int64_t m, const int* label, uint32_t* klo,
-                             uint32_t* khi, uint32_t* order, cudaStream_t s) {
-    if (m == 0) return cudaSuccess;
-    ++g_launches;
-    dual_keys_kernel<<<nblk(m), 256, 0, s>>>(tri, faces, m, label, klo, khi, order);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_gather_u32(const uint32_t* src, const uint32_t* idx, int64_t m, uint32_t* dst, cudaStream_t s) {
-    if (m == 0) return cudaSuccess;
-    ++g_launches;
-    gather_u32_kernel<<<nblk(m), 256, 0, s>>>(src, idx, m, dst);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_dual_unique(const uint32_t* klo, const uint32_t* khi, const uint32_t* order, int64_t m,
-                               uint32_t* keep, cudaStream_t s) {
-    if (m == 0) return cudaSuccess;
-    ++g_launches;
-    dual_unique_kernel<<<nblk(m), 256, 0, s>>>(klo, khi, order, m, keep);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_dual_write(const int* tri, const int* faces, const int* sel, int64_t t, const int* label,
-                              int* out, cudaStream_t s) {
-    if (t == 0) return cudaSuccess;
-    ++g_launches;
-    dual_write_kernel<<<nblk(t), 256, 0, s>>>(tri, faces, sel, t, label, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_centroids(int metric, const DevState& st, double* out, cudaStream_t s) {
-    if (st.k == 0) return cudaSuccess;
-    ACVD_DISPATCH(metric, centroids_kernel, nblk(st.k), 256, s, st, out);
     return cudaGetLastError();
 }
 

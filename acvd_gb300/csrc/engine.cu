@@ -136,6 +136,10 @@ struct acvd_ctx {
     DBuf<unsigned long long> best;
     DBuf<double> dtmp;
     Scratch scratch;
+    // outputs on their way to the host, kept between calls
+    DBuf<double> cl_out, wk_quad;
+    DBuf<int> wk_ids, wk_dual;
+    DBuf<char> wk_hash;
 
     // sweep graph; one event pair per colour class brackets its evaluation kernel
     cudaGraphExec_t sweep_exec = nullptr;
@@ -964,12 +968,13 @@ static int group_by_cluster(acvd_ctx* ctx, const DevState& st) {
     return ACVD_OK;
 }
 
-static int recompute(acvd_ctx* ctx) {
+// Sums, records and energies of the current clustering; `out`: device outputs written along.
+static int recompute(acvd_ctx* ctx, const ClusterOut& out = ClusterOut()) {
     DevState st = ctx->state();
     const int r = group_by_cluster(ctx, st);
     if (r) return r;
     CK(launch_reduce_clusters(ctx->metric, st, ctx->wk_b.p, ctx->wk_off.p, ctx->s));
-    CK(launch_update_all(ctx->metric, st, ctx->s));
+    CK(launch_update_all(ctx->metric, st, out, ctx->s));
     return ACVD_OK;
 }
 
@@ -1662,46 +1667,30 @@ extern "C" int acvd_get_clusters(acvd_ctx* ctx, int32_t* sizes, double* S, doubl
     ctx->flags.level = ctx->level;
     int r = upload_flags(ctx);
     if (r) return r;
-    r = recompute(ctx);
-    if (r) return r;
-    const int K = ctx->K;
-    const int as = acc_stride(ctx->metric);
-    // the accumulators come back only when one of their views is asked for
-    const bool want_acc = S || W || quadric;
-    std::vector<df> acc(want_acc ? (size_t)K * as : 0);
-    if (want_acc)
-        CK(cudaMemcpyAsync(acc.data(), ctx->acc.p, acc.size() * sizeof(df), cudaMemcpyDeviceToHost, ctx->s));
-    if (sizes) CK(cudaMemcpyAsync(sizes, ctx->size.p, K * sizeof(int), cudaMemcpyDeviceToHost, ctx->s));
-    if (energy) CK(cudaMemcpyAsync(energy, ctx->energy.p, K * sizeof(double), cudaMemcpyDeviceToHost, ctx->s));
+    const size_t K = ctx->K;
+    CK(ctx->cl_out.resize(16 * K));
+    ClusterOut out;
+    double* p = ctx->cl_out.p;
+    if (S) { out.S = p; p += 3 * K; }
+    if (W) { out.W = p; p += K; }
+    if (quadric) { out.Q = p; p += 9 * K; }
+    if (centroid) out.centroid = p;
+    if ((r = recompute(ctx, out))) return r;
+    auto back = [&](void* to, const void* from, size_t bytes) {
+        return to ? cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, ctx->s) : cudaSuccess;
+    };
     if (energy_total) {
         CK(ctx->dtmp.resize(2));
-        CK(sum_f64(ctx->energy.p, K, ctx->dtmp.p, ctx->scratch, ctx->s));
-        CK(cudaMemcpyAsync(energy_total, ctx->dtmp.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->s));
+        CK(sum_f64(ctx->energy.p, ctx->K, ctx->dtmp.p, ctx->scratch, ctx->s));
     }
-    if (centroid) {
-        DBuf<double> c;
-        CK(c.resize(3 * (size_t)K));
-        CK(launch_centroids(ctx->metric, ctx->state(), c.p, ctx->s));
-        CK(cudaMemcpyAsync(centroid, c.p, 3 * (size_t)K * sizeof(double), cudaMemcpyDeviceToHost, ctx->s));
-        CK(cudaStreamSynchronize(ctx->s));
-    }
+    CK(back(S, out.S, 3 * K * sizeof(double)));
+    CK(back(W, out.W, K * sizeof(double)));
+    CK(back(quadric, out.Q, 9 * K * sizeof(double)));
+    CK(back(centroid, out.centroid, 3 * K * sizeof(double)));
+    CK(back(sizes, ctx->size.p, K * sizeof(int)));
+    CK(back(energy, ctx->energy.p, K * sizeof(double)));
+    CK(back(energy_total, ctx->dtmp.p, sizeof(double)));
     CK(cudaStreamSynchronize(ctx->s));
-    for (int k = 0; want_acc && k < K; k++) {
-        const df* a = acc.data() + (size_t)k * as;
-        auto d = [](df x) { return (double)x.hi + (double)x.lo; };
-        if (S) for (int j = 0; j < 3; j++) S[3 * k + j] = d(a[j]);
-        if (W) W[k] = d(a[3]);
-        if (quadric) {
-            double* q = quadric + 9 * (size_t)k;
-            if (ctx->metric == kIso) {
-                for (int j = 0; j < 9; j++) q[j] = 0.0;
-            } else {
-                // the reference's compact quadric: A entries and -b in slots 3, 6, 8
-                q[0] = d(a[4]); q[1] = d(a[5]); q[2] = d(a[6]); q[3] = -d(a[10]);
-                q[4] = d(a[7]); q[5] = d(a[8]); q[6] = -d(a[11]); q[7] = d(a[9]); q[8] = -d(a[12]);
-            }
-        }
-    }
     return ACVD_OK;
 }
 
@@ -1727,22 +1716,19 @@ extern "C" int acvd_get_boundary_edges(acvd_ctx* ctx, int32_t* ids, int64_t* cou
     if (!ctx->ready_labels) return fail(ctx, ACVD_ERR_ARG, "no labels");
     CK(cudaSetDevice(ctx->opts.device));
     const int64_t ne = ctx->nE;
-    DBuf<uint32_t> flags, pos;
-    DBuf<int> out;
-    CK(flags.resize(ne + 1));
-    CK(pos.resize(ne + 1));
+    const size_t words = boundary_edges_scratch(ne);
+    CK(ctx->wk_ids.resize(ne));
+    CK(ctx->scratch.reserve(words * sizeof(uint32_t)));
     CK(ctx->dtmp.resize(2));
     uint32_t* total = (uint32_t*)ctx->dtmp.p;
-    CK(launch_boundary_edges(ctx->edge_int.p, ne, ctx->label.p, flags.p, ctx->s));
-    CK(exclusive_scan_u32(flags.p, pos.p, ne, total, ctx->scratch, ctx->s));
+    CK(launch_boundary_edges(ctx->edge_int.p, ne, ctx->label.p, ctx->wk_ids.p, total, (uint32_t*)ctx->scratch.ptr, words,
+                             ctx->s));
     uint32_t t = 0;
     CK(cudaMemcpyAsync(&t, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->s));
     CK(cudaStreamSynchronize(ctx->s));
     *count = t;
     if (ids && t) {
-        CK(out.resize(t));
-        CK(launch_compact(flags.p, pos.p, ne, out.p, ctx->s));
-        CK(cudaMemcpyAsync(ids, out.p, t * sizeof(int), cudaMemcpyDeviceToHost, ctx->s));
+        CK(cudaMemcpyAsync(ids, ctx->wk_ids.p, t * sizeof(int), cudaMemcpyDeviceToHost, ctx->s));
         CK(cudaStreamSynchronize(ctx->s));
     }
     return ACVD_OK;
@@ -1879,79 +1865,54 @@ extern "C" int acvd_post_placement(acvd_ctx* ctx, int level, double* points) {
     ctx->flags.level = ctx->level;
     int r = upload_flags(ctx);
     if (r) return r;
-    r = recompute(ctx);
-    if (r) return r;
     const int64_t nv = ctx->nV;
     const int K = ctx->K;
     // the output vertices before placement: the metric's cluster centroids
-    DBuf<double> start, qv, out;
-    CK(start.resize(3 * (size_t)K));
-    CK(launch_centroids(ctx->metric, ctx->state(), start.p, ctx->s));
+    CK(ctx->cl_out.resize(16 * (size_t)K));
+    ClusterOut start;
+    start.centroid = ctx->cl_out.p;
+    if ((r = recompute(ctx, start))) return r;
+    double* out = ctx->cl_out.p + 3 * (size_t)K;
     // items by cluster, in original vertex ids
     CK(ctx->label_orig.resize(nv));
     CK(launch_gather_i32(ctx->label.p, ctx->inv.p, nv, ctx->label_orig.p, ctx->s));
     DevState st = ctx->state();
     st.label = ctx->label_orig.p;
     if ((r = group_by_cluster(ctx, st))) return r;
-    CK(qv.resize(9 * (size_t)nv));
-    CK(launch_vertex_quadrics(ctx->xyz.p, ctx->tri.p, ctx->vf_row.p, ctx->vf_face.p, nv, qv.p, ctx->s));
-    CK(out.resize(3 * (size_t)K));
+    CK(ctx->wk_quad.resize(9 * (size_t)nv));
+    CK(launch_vertex_quadrics(ctx->xyz.p, ctx->tri.p, ctx->vf_row.p, ctx->vf_face.p, nv, ctx->wk_quad.p, ctx->s));
     CK(ctx->dtmp.resize(2));
-    CK(launch_post_place(qv.p, ctx->wk_b.p, ctx->wk_off.p, (int*)ctx->dtmp.p, start.p, K, level, out.p, ctx->s));
-    CK(cudaMemcpyAsync(points, out.p, 3 * (size_t)K * sizeof(double), cudaMemcpyDeviceToHost, ctx->s));
+    CK(launch_post_place(ctx->wk_quad.p, ctx->wk_b.p, ctx->wk_off.p, (int*)ctx->dtmp.p, start.centroid, K, level, out,
+                         ctx->s));
+    CK(cudaMemcpyAsync(points, out, 3 * (size_t)K * sizeof(double), cudaMemcpyDeviceToHost, ctx->s));
     CK(cudaStreamSynchronize(ctx->s));
     return ACVD_OK;
 }
 
-// The dual mesh's triangles on the device (cluster ids), *n_tris of them in `out`.
-static int build_dual(acvd_ctx* ctx, DBuf<int>& out, int64_t* n_tris) {
+// The dual mesh's triangles on the device (cluster ids), *n_tris of them in wk_dual.  The
+// hash table has 8 slots per cluster (a closed surface has about 2 triangles per vertex),
+// or, for a labelling with many more label sets, two per face.
+static int build_dual(acvd_ctx* ctx, int64_t* n_tris) {
     const int64_t nf = ctx->nF;
-    DBuf<uint32_t> flags, pos, klo, khi, order, t1, t2, keep, kpos;
-    DBuf<int> faces, sel;
-    CK(flags.resize(nf + 1));
-    CK(pos.resize(nf + 1));
+    int64_t most = 4096, slots = 4096;
+    while (most < 2 * nf) most *= 2;
+    while (slots < 8 * (int64_t)ctx->K) slots *= 2;
+    slots = std::min(slots, most);
     CK(ctx->dtmp.resize(2));
-    uint32_t* total = (uint32_t*)ctx->dtmp.p;
-    CK(launch_dual_faces(ctx->tri_int.p, nf, ctx->label.p, ctx->K, flags.p, ctx->s));
-    CK(exclusive_scan_u32(flags.p, pos.p, nf, total, ctx->scratch, ctx->s));
-    uint32_t m = 0;
-    CK(cudaMemcpyAsync(&m, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->s));
-    CK(cudaStreamSynchronize(ctx->s));
-    if (m == 0) { *n_tris = 0; return ACVD_OK; }
-    CK(faces.resize(m));
-    CK(launch_compact(flags.p, pos.p, nf, faces.p, ctx->s));
-    CK(klo.resize(m)); CK(khi.resize(m)); CK(order.resize(m)); CK(t1.resize(m)); CK(t2.resize(m));
-    CK(keep.resize(m + 1)); CK(kpos.resize(m + 1));
-    CK(launch_dual_keys(ctx->tri_int.p, faces.p, m, ctx->label.p, klo.p, khi.p, order.p, ctx->s));
-    // stable LSD sort on (khi, klo): by klo first, then by khi
-    CK(radix_sort_pairs(klo.p, order.p, t1.p, t2.p, m, 32, ctx->scratch, ctx->s));
-    CK(launch_gather_u32(khi.p, order.p, m, t1.p, ctx->s));           // khi in klo-sorted order
-    CK(cudaMemcpyAsync(khi.p, t1.p, m * sizeof(uint32_t), cudaMemcpyDeviceToDevice, ctx->s));
-    // carry klo along the second pass through a permutation index
-    DBuf<uint32_t> perm, klo2;
-    CK(perm.resize(m)); CK(klo2.resize(m));
-    {
-        std::vector<uint32_t> io(m);
-        for (uint32_t j = 0; j < m; j++) io[j] = j;
-        CK(cudaMemcpyAsync(perm.p, io.data(), m * sizeof(uint32_t), cudaMemcpyHostToDevice, ctx->s));
+    unsigned* d_got = (unsigned*)ctx->dtmp.p;
+    for (;;) {
+        CK(ctx->wk_hash.resize(dual_work_bytes(nf, slots)));
+        CK(ctx->wk_dual.resize(3 * (size_t)std::min(nf, slots)));
+        CK(launch_dual(ctx->tri_int.p, nf, ctx->label.p, ctx->K, slots, slots == most ? (unsigned)most : 64u,
+                       ctx->wk_hash.p, ctx->wk_dual.p, d_got, ctx->s));
+        unsigned got[2];
+        CK(cudaMemcpyAsync(got, d_got, sizeof got, cudaMemcpyDeviceToHost, ctx->s));
         CK(cudaStreamSynchronize(ctx->s));
+        *n_tris = got[0];
+        if (!got[1]) return ACVD_OK;
+        if (slots == most) return fail(ctx, ACVD_ERR_DEVICE_CHECK, "dual mesh: the label sets do not fit their table");
+        slots = most;
     }
-    CK(radix_sort_pairs(khi.p, perm.p, t1.p, t2.p, m, 31, ctx->scratch, ctx->s));
-    CK(launch_gather_u32(klo.p, perm.p, m, klo2.p, ctx->s));
-    CK(launch_gather_u32(order.p, perm.p, m, t1.p, ctx->s));
-    CK(launch_dual_unique(klo2.p, khi.p, t1.p, m, keep.p, ctx->s));
-    CK(exclusive_scan_u32(keep.p, kpos.p, m, total, ctx->scratch, ctx->s));
-    uint32_t t = 0;
-    CK(cudaMemcpyAsync(&t, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->s));
-    CK(cudaStreamSynchronize(ctx->s));
-    *n_tris = t;
-    if (t) {
-        CK(sel.resize(t));
-        CK(out.resize(3 * (size_t)t));
-        CK(launch_compact(keep.p, kpos.p, m, sel.p, ctx->s));
-        CK(launch_dual_write(ctx->tri_int.p, faces.p, sel.p, t, ctx->label.p, out.p, ctx->s));
-    }
-    return ACVD_OK;
 }
 
 // One pass of vtkDiscreteRemeshing::DetectNonManifoldOutputVertices
@@ -1970,9 +1931,9 @@ extern "C" int acvd_force_manifold_step(acvd_ctx* ctx, int32_t* n_issues, int32_
     *n_clusters = ctx->K;
     int r = recompute(ctx);   // current cluster sizes
     if (r) return r;
-    DBuf<int> dt;
     int64_t t = 0;
-    if ((r = build_dual(ctx, dt, &t))) return r;
+    if ((r = build_dual(ctx, &t))) return r;
+    const DBuf<int>& dt = ctx->wk_dual;
     const int K = ctx->K;
     const int64_t nv = ctx->nV, ne = ctx->nE;
     DBuf<unsigned> cnt, off, cursor;
@@ -2225,13 +2186,12 @@ extern "C" int acvd_get_dual_mesh(acvd_ctx* ctx, int32_t* tris, int64_t* n_tris)
     if (!ctx || !n_tris) return ACVD_ERR_ARG;
     if (!ctx->ready_labels) return fail(ctx, ACVD_ERR_ARG, "no labels");
     CK(cudaSetDevice(ctx->opts.device));
-    DBuf<int> out;
     int64_t t = 0;
-    const int r = build_dual(ctx, out, &t);
+    const int r = build_dual(ctx, &t);
     if (r) return r;
     *n_tris = t;
     if (tris && t) {
-        CK(cudaMemcpyAsync(tris, out.p, 3 * (size_t)t * sizeof(int), cudaMemcpyDeviceToHost, ctx->s));
+        CK(cudaMemcpyAsync(tris, ctx->wk_dual.p, 3 * (size_t)t * sizeof(int), cudaMemcpyDeviceToHost, ctx->s));
         CK(cudaStreamSynchronize(ctx->s));
     }
     return ACVD_OK;

@@ -12,6 +12,7 @@
 #include "../../include/acvd_gpu.h"
 #include "common.cuh"
 #include "primitives.cuh"
+#include "state.cuh"
 
 // 256 KiB: tile counts (one word per 2048 edges) plus the scan's partial sums
 // for the largest accepted input.  Every word a call reads is written by the
@@ -103,6 +104,25 @@ int na_scratch(uint32_t** out) {
 }
 
 }  // namespace
+
+size_t boundary_edges_scratch(int64_t ne) {
+    const int64_t nb = ne > 0 ? (ne + kNaTile - 1) / kNaTile : 1;
+    return (size_t)nb + scan_scratch_need(nb);
+}
+
+cudaError_t launch_boundary_edges(const int* edge_v, int64_t ne, const int* label, int* ids, uint32_t* count,
+                                  uint32_t* scratch, size_t scratch_words, cudaStream_t s) {
+    const int64_t nb = ne > 0 ? (ne + kNaTile - 1) / kNaTile : 1;
+    ++g_launches;
+    na_count_kernel<<<(unsigned)nb, kNaThreads, 0, s>>>(edge_v, ne, label, scratch);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = exclusive_scan_u32_raw(scratch, scratch, nb, scratch + nb, scratch_words - (size_t)nb, s);
+    if (e != cudaSuccess) return e;
+    ++g_launches;
+    na_compact_kernel<<<(unsigned)nb, kNaThreads, 0, s>>>(edge_v, ne, label, scratch, ids, count);
+    return cudaGetLastError();
+}
+
 }  // namespace acvd
 
 extern "C" int acvd_boundary_edges_noalloc(const int32_t* d_edge_v, int64_t n_edges, const int32_t* d_labels,
@@ -116,18 +136,9 @@ extern "C" int acvd_boundary_edges_noalloc(const int32_t* d_edge_v, int64_t n_ed
     uint32_t* scratch = nullptr;
     const int rc = na_scratch(&scratch);
     if (rc != ACVD_OK) return rc;
-    const int64_t nb = n_edges > 0 ? (n_edges + kNaTile - 1) / kNaTile : 1;
-    const size_t need = (size_t)nb + scan_scratch_need(nb);
-    if (need > kNoAllocScratchWords) return ACVD_ERR_UNSUPPORTED;
-    cudaStream_t s = (cudaStream_t)stream;
-    uint32_t* tile = scratch;
-    ++g_launches;
-    na_count_kernel<<<(unsigned)nb, kNaThreads, 0, s>>>(d_edge_v, n_edges, d_labels, tile);
-    if (cudaGetLastError() != cudaSuccess) return ACVD_ERR_CUDA;
-    if (exclusive_scan_u32_raw(tile, tile, nb, scratch + nb, kNoAllocScratchWords - (size_t)nb, s) != cudaSuccess)
-        return ACVD_ERR_CUDA;
-    ++g_launches;
-    na_compact_kernel<<<(unsigned)nb, kNaThreads, 0, s>>>(d_edge_v, n_edges, d_labels, tile, d_ids, d_count);
-    if (cudaGetLastError() != cudaSuccess) return ACVD_ERR_CUDA;
-    return ACVD_OK;
+    if (boundary_edges_scratch(n_edges) > kNoAllocScratchWords) return ACVD_ERR_UNSUPPORTED;
+    return launch_boundary_edges(d_edge_v, n_edges, d_labels, d_ids, d_count, scratch, kNoAllocScratchWords,
+                                 (cudaStream_t)stream) == cudaSuccess
+               ? ACVD_OK
+               : ACVD_ERR_CUDA;
 }

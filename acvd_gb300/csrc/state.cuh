@@ -347,7 +347,15 @@ cudaError_t launch_reclaim(const DevState& st, int item0, int64_t count, int col
 // blocks per SM for this metric (0 when the kernel cannot be co-resident).
 int sweep_run_blocks_per_sm(int metric);
 cudaError_t launch_sweep_run(int metric, const SweepRun& a, int grid, cudaStream_t s);
-cudaError_t launch_update_all(int metric, const DevState& st, cudaStream_t s);
+// device outputs of acvd_get_clusters, any may be null: S (3 k), W (k), the compact quadric (9 k)
+// and the FP64 placed vertices (3 k)
+struct ClusterOut {
+    double* S = nullptr;
+    double* W = nullptr;
+    double* Q = nullptr;
+    double* centroid = nullptr;
+};
+cudaError_t launch_update_all(int metric, const DevState& st, const ClusterOut& out, cudaStream_t s);
 cudaError_t launch_cluster_keys(const DevState& st, uint32_t* keys, uint32_t* vals, cudaStream_t s);
 // cluster c's items at sorted_items[seg_off[c] .. seg_off[c + 1])
 cudaError_t launch_reduce_clusters(int metric, const DevState& st, const uint32_t* sorted_items,
@@ -369,23 +377,26 @@ cudaError_t launch_fill_list(const DevState& st, const int* list, const unsigned
 // items; *err = 1 if the round bound ran out, 2 if the lists were longer (nothing done)
 cudaError_t launch_fill_block(const DevState& st, const int* list, const int64_t* off, int ncolors,
                               const unsigned* cnt, unsigned* err, unsigned max_items, cudaStream_t s);
-cudaError_t launch_boundary_edges(const int* edge_v, int64_t ne, const int* label, uint32_t* flags,
-                                  cudaStream_t s);
 cudaError_t launch_compact(const uint32_t* flags, const uint32_t* pos, int64_t n, int* out, cudaStream_t s);
-cudaError_t launch_dual_faces(const int* tri, int64_t nf, const int* label, int k, uint32_t* flags,
-                              cudaStream_t s);
-cudaError_t launch_dual_keys(const int* tri, const int* faces, int64_t m, const int* label, uint32_t* klo,
-                             uint32_t* khi, uint32_t* order, cudaStream_t s);
-cudaError_t launch_gather_u32(const uint32_t* src, const uint32_t* idx, int64_t m, uint32_t* dst, cudaStream_t s);
-cudaError_t launch_dual_unique(const uint32_t* klo, const uint32_t* khi, const uint32_t* order, int64_t m,
-                               uint32_t* keep, cudaStream_t s);
-cudaError_t launch_dual_write(const int* tri, const int* faces, const int* sel, int64_t t, const int* label,
-                              int* out, cudaStream_t s);
-cudaError_t launch_centroids(int metric, const DevState& st, double* out, cudaStream_t s);
 cudaError_t launch_vertex_quadrics(const double* xyz, const int* tri, const uint32_t* vf_row, const uint32_t* vf_face,
                                    int64_t nv, double* qv, cudaStream_t s);
 cudaError_t launch_post_place(const double* qv, const uint32_t* sorted, const uint32_t* seg_off, int* first,
                               const double* start, int k, int level, double* out, cudaStream_t s);
+
+// ---- dual mesh (dual.cu) ----
+// tri: faces in item ids; slots: hash slots, a power of two of at least 4; probes: steps a
+// label set may take to find its slot; work: dual_work_bytes; out: 3 * min(nf, slots) ints;
+// total_full[0]: triangles written, [1]: nonzero when the table was too full (no result)
+size_t dual_work_bytes(int64_t nf, int64_t slots);
+cudaError_t launch_dual(const int* tri, int64_t nf, const int* label, int k, int64_t slots, unsigned probes,
+                        void* work, int* out, unsigned* total_full, cudaStream_t s);
+
+// ---- boundary edges of a labelling (noalloc.cu) ----
+// edge ids whose ends carry different labels, increasing, and their number in *count;
+// scratch: boundary_edges_scratch(ne) words
+size_t boundary_edges_scratch(int64_t ne);
+cudaError_t launch_boundary_edges(const int* edge_v, int64_t ne, const int* label, int* ids, uint32_t* count,
+                                  uint32_t* scratch, size_t scratch_words, cudaStream_t s);
 
 // ---- curvature (curvature.cu) ----
 size_t curvature_face_bytes(int64_t nf);

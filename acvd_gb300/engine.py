@@ -533,15 +533,15 @@ class Engine:
                 "energy": E, "energy_total": tot.value}
 
     def boundary_edges(self) -> np.ndarray:
+        # one call into a buffer of the largest size (untouched pages cost nothing), cut to what came
         n = _i64()
-        self._ck(self._lib.acvd_get_boundary_edges(self.ctx, None, ctypes.byref(n)))
-        out = np.empty(max(n.value, 1), dtype=np.int32)
+        out = np.empty(max(self.n_edges, 1), dtype=np.int32)
         self._ck(self._lib.acvd_get_boundary_edges(self.ctx, _ptr(out), ctypes.byref(n)))
-        return out[:n.value]
+        return out[:n.value].copy()
 
     def dual_mesh(self) -> np.ndarray:
         n = _i64()
-        self._ck(self._lib.acvd_get_dual_mesh(self.ctx, None, ctypes.byref(n)))
-        out = np.empty(3 * max(n.value, 1), dtype=np.int32)
+        faces = self._tri.shape[0] if self.n else 0
+        out = np.empty(3 * max(faces, 1), dtype=np.int32)
         self._ck(self._lib.acvd_get_dual_mesh(self.ctx, _ptr(out), ctypes.byref(n)))
-        return out[:3 * n.value].reshape(-1, 3)
+        return out[:3 * n.value].reshape(-1, 3).copy()

@@ -22,6 +22,7 @@
 // decompositions 62 -> 42-55 us; forward and backward together 1.25 -> 0.63 ms.
 #include <cmath>
 
+#include "common.cuh"
 #include "primitives.cuh"
 #include "state.cuh"
 
@@ -32,12 +33,6 @@ ACVD_DEV void get2(const double* p, double& a, double& b) {
     const double2 v = *reinterpret_cast<const double2*>(p);
     a = v.x;
     b = v.y;
-}
-
-// a / b from inv = 1 / b: one exact-residual correction of the product (Markstein 1990)
-ACVD_DEV double quotient(double a, double b, double inv) {
-    const double q = a * inv;
-    return fma(fma(-b, q, a), inv, q);
 }
 
 // r^g; the exponents of a plain density and of none need no power

@@ -3,11 +3,24 @@
 // vtkCurvatureMeasure (DiscreteRemeshing/vtkDiscreteRemeshing.h:630-637):
 // polynomial fitting (method 1) on the faces of the vertex 3-ring.
 //
-// One thread per vertex, FP64.  This file is compiled without FMA contraction
+// FP64, one thread per vertex.  This file is compiled without FMA contraction
 // (build.py) and every expression keeps the operation order of the CPU
 // restatement, so that each value equals it bit for bit (the divisions and
 // square roots are the correctly rounded IEEE operations on both sides).
+//
+// What bounds it: the FP64 pipe, 2 lanes per SM and cycle.  A vertex's fit reads its 3-ring's
+// faces (54 in a regular mesh) three times, about 100 FP64 operations a face and 800 for the
+// 6 x 6 inverse: 5.3 ms for 524,288 vertices at that rate.  So
+//  * products that depend on the face only are formed once per face;
+//  * quotients by one divisor (five per face, 51 per inverse) share its reciprocal
+//    (quotient(): 3 operations instead of about 9);
+//  * finding the 3-ring, integer work in dependent loads, has kernels of its own at their own
+//    occupancy instead of idling the FP64 pipe in between: every vertex's fan of faces
+//    once, then the list of each vertex's ring, in chunks of kCurvChunk vertices.
+// 6.46 ms of fits and 0.76 of lists for 524,288 vertices; one kernel for both, with 8,500 FP64
+// operations per vertex, took 9.9 ms with its pipe 72 % busy.
 #include "../../include/acvd_gpu.h"
+#include "common.cuh"
 #include "primitives.cuh"
 #include "state.cuh"
 
@@ -16,6 +29,18 @@ namespace acvd {
 constexpr int kCurvMaxF = 192;    // faces of one 3-ring
 constexpr int kCurvMaxV = 384;    // vertices queued for one ring step
 constexpr int kCurvMaxVis = 96;   // vertices of rings 0..2
+// vertices whose face lists are held at a time (up to 403 MB): enough blocks for the last
+// wave not to show
+constexpr int64_t kCurvChunk = 1 << 19;
+
+constexpr int kFitBatch = 4;
+
+// whether 1 / b and quotients of such numbers by b stay in the normal range: 2^-465 <= |b| <
+// 2^465, read off the exponent (a comparison in FP64 runs on the pipe that bounds it all)
+__device__ __forceinline__ bool divides_well(double b) {
+    return (((unsigned)__double2hiint(b) >> 20) & 0x7ffu) - 558u < 930u;
+}
+__device__ __forceinline__ bool divided_well(double a) { return divides_well(a) || __double_as_longlong(a) << 1 == 0; }
 
 // Faces of edge e: the first two faces, in increasing id, holding both of its
 // endpoints (the reference attaches faces to an edge in face order,
@@ -49,26 +74,22 @@ __global__ void slot_edges_kernel(const int* __restrict__ edge_int, int64_t ne, 
         if (col[p] == a) { slot_edge[p] = (int)e; break; }
 }
 
-// Per face, once: unit normal, area and area-weighted barycentre, the values the
-// fit reads for every vertex whose 3-ring holds the face.
+// Per face, once: the values the fit reads for every vertex whose 3-ring holds the face.
 struct FaceProps {
-    double n[3];
+    double an[3];     // area x unit normal
+    double ab[3];     // area x barycentre
     double area;
-    double bary[3];
-    double pad;
+    double bary[3];   // area-weighted barycentre
 };
 
 struct CurvMesh {
-    const double* xyz;
-    const int* tri;
     const FaceProps* fp;
     int64_t nv;
-    const int* row;        // internal ring CSR
+    const int* row;         // internal ring CSR
     const int* col;
-    const int* perm;       // item -> original vertex
-    const int* inv;        // original vertex -> item
-    const int* slot_edge;
-    const int2* poly;
+    const int* inv;         // original vertex -> item
+    const int* fan;         // per item: the faces of its ring edges, each once, at 2 row[i]
+    const int* fan_count;
 };
 
 // area by the side-length form (Common/vtkSurface.cxx:1283) and the
@@ -82,10 +103,17 @@ __device__ void curv_face_mass(const double p1[3], const double p2[3], const dou
     const double b = d23[0] * d23[0] + d23[1] * d23[1] + d23[2] * d23[2];
     const double c = d31[0] * d31[0] + d31[1] * d31[1] + d31[2] * d31[2];
     const double a2 = 0.25 * sqrt(fabs(4.0 * a * c - (a - b + c) * (a - b + c)));
-    for (int i = 0; i < 3; i++) bary[i] = 0.0 + a2 * (p1[i] + p2[i] + p3[i]) / 3.0;
+    for (int i = 0; i < 3; i++) {
+        const double t = a2 * (p1[i] + p2[i] + p3[i]);
+        bary[i] = 0.0 + (divided_well(t) ? quotient(t, 3.0, 1.0 / 3.0) : t / 3.0);
+    }
     area = 0.0 + a2;
-    if (area > 0)
+    if (divides_well(area)) {
+        const double inv = 1.0 / area;
+        for (int i = 0; i < 3; i++) bary[i] = divided_well(bary[i]) ? quotient(bary[i], area, inv) : bary[i] / area;
+    } else if (area > 0) {
         for (int i = 0; i < 3; i++) bary[i] /= area;
+    }
 }
 
 // unit normal from (x3 - x2) x (x1 - x2)
@@ -96,7 +124,12 @@ __device__ void curv_normal(const double x1[3], const double x2[3], const double
     n[1] = a[2] * b[0] - a[0] * b[2];
     n[2] = a[0] * b[1] - a[1] * b[0];
     const double l = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
-    if (l != 0.0) { n[0] /= l; n[1] /= l; n[2] /= l; }
+    if (divides_well(l)) {
+        const double inv = 1.0 / l;
+        for (int k = 0; k < 3; k++) n[k] = divided_well(n[k]) ? quotient(n[k], l, inv) : n[k] / l;
+    } else if (l != 0.0) {
+        n[0] /= l; n[1] /= l; n[2] /= l;
+    }
 }
 
 __device__ __forceinline__ void curv_normalize(double a[3]) {
@@ -124,17 +157,150 @@ __global__ void face_props_kernel(const double* __restrict__ xyz, const int* __r
         p3[k] = xyz[3 * (int64_t)tri[3 * f + 2] + k];
     }
     FaceProps r;
-    curv_normal(p1, p2, p3, r.n);
+    double n[3];
+    curv_normal(p1, p2, p3, n);
     curv_face_mass(p1, p2, p3, r.area, r.bary);
-    r.pad = 0.0;
+    for (int k = 0; k < 3; k++) {
+        r.an[k] = r.area * n[k];
+        r.ab[k] = r.area * r.bary[k];
+    }
     fp[f] = r;
+}
+
+// The faces around item i in the order its ring's edges name them (each edge's first two
+// faces), each once: the order in which vtkNeighbourhoodComputation meets them.
+__global__ void fan_kernel(int64_t n, const int* __restrict__ row, const int* __restrict__ slot_edge,
+                           const int2* __restrict__ poly, int* fan, int* __restrict__ fan_count) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int p0 = row[i], p1 = row[i + 1];
+    int* out = fan + 2 * (int64_t)p0;
+    int c = 0;
+    auto add = [&](int f) {
+        for (int j = 0; j < c; j++)
+            if (out[j] == f) return;
+        out[c++] = f;
+    };
+    for (int p = p0; p < p1; p++) {
+        const int e = slot_edge[p];
+        if (e < 0) continue;
+        const int2 pf = poly[e];
+        if (pf.x >= 0) add(pf.x);
+        if (pf.y >= 0) add(pf.y);
+    }
+    fan_count[i] = c;
+}
+
+// The faces of the 3-ring of vertices v0 .. v0 + n - 1 in the reference's order
+// (vtkNeighbourhoodComputation::ComputeNRingCells, Common/vtkNeighbourhoodComputation.cxx:38-100:
+// the vertex's own faces, then ring by ring the faces of each vertex not yet visited):
+// lists[j * n + t] is the j-th face of vertex v0 + t, so that a warp's accesses to a place of
+// its lists fall side by side.
+// counts[t]: their number, -1 for a neighbourhood larger than the bounds above, which also
+// counts in *overflow.
+//
+// kRingLanes lanes work on a vertex: its lists are in shared memory, a visited vertex's fan
+// is looked up in them one face per lane, a ring's vertices likewise.  A thread per vertex left
+// 1,281 warps with a chain of 63,000 instructions each for 40,962 vertices: 465 us, 71 so
+// (524,288 vertices of a grid, where both are bound by instructions: 576 and 755 us).
+constexpr int kRingThreads = 128;
+constexpr int kRingLanes = 8;
+constexpr int kRingGroups = kRingThreads / kRingLanes;
+
+__global__ void __launch_bounds__(kRingThreads) ring_faces_kernel(CurvMesh m, int64_t v0, int64_t n,
+                                                                  int* __restrict__ lists, int* __restrict__ counts,
+                                                                  unsigned long long* __restrict__ overflow) {
+    // rows of 4 (mod 32) words: the groups of a warp in different banks; -1 where nothing is listed,
+    // so that a search may take four entries at a time
+    __shared__ __align__(16) int s_fl[kRingGroups][kCurvMaxF + 4];
+    __shared__ __align__(16) int s_vis[kRingGroups][kCurvMaxVis + 4];
+    __shared__ int s_nf[kRingGroups];
+    const int g = threadIdx.x / kRingLanes, l = threadIdx.x % kRingLanes;
+    const int shift = (threadIdx.x & 31) & ~(kRingLanes - 1);   // the group's first lane in the warp
+    const unsigned group = ((1u << kRingLanes) - 1u) << shift;
+    const int64_t t0 = (int64_t)blockIdx.x * kRingGroups, t = t0 + g;
+    int* fl = s_fl[g];
+    int* vis = s_vis[g];
+    for (int i = l; i < kCurvMaxF + 4; i += kRingLanes) fl[i] = -1;
+    for (int i = l; i < kCurvMaxVis + 4; i += kRingLanes) vis[i] = -1;
+    __syncwarp();
+    // whether x is none of the first c entries of a list
+    auto absent = [](const int* list, int c, int x) {
+        bool none = true;
+        for (int i = 0; i < c; i += 4) {
+            const int4 q = *reinterpret_cast<const int4*>(list + i);
+            none = none && q.x != x && q.y != x && q.z != x && q.w != x;
+        }
+        return none;
+    };
+    int nf = 0, nvis = 0;
+    bool ok = true;
+    // u joins the visited vertices; the faces of its fan that are not listed follow in order
+    auto visit = [&](int u, int& queued) {
+        if (nvis == kCurvMaxVis) { ok = false; return; }
+        if (l == 0) vis[nvis] = u;
+        nvis++;
+        const int p0 = m.row[u], p1 = m.row[u + 1], c = m.fan_count[u];
+        queued += p1 - p0;
+        if (queued > kCurvMaxV) { ok = false; return; }
+        const int* fan = m.fan + 2 * (int64_t)p0;
+        for (int k0 = 0; k0 < c; k0 += kRingLanes) {
+            const int f = k0 + l < c ? fan[k0 + l] : -1;
+            const bool fresh = absent(fl, nf, f) && f >= 0;
+            const unsigned add = (__ballot_sync(group, fresh) & group) >> shift;
+            if (nf + __popc(add) > kCurvMaxF) { ok = false; return; }
+            if (fresh) fl[nf + __popc(add & ((1u << l) - 1u))] = f;
+            nf += __popc(add);
+            __syncwarp(group);
+        }
+        __syncwarp(group);
+    };
+    if (t < n) {
+        int queued = 0;
+        visit(m.inv[v0 + t], queued);
+        // ring r's new vertices are vis[first .. last); the next ring's candidates are their
+        // neighbours in order
+        int first = 0, last = nvis;
+        for (int r = 1; r < 3 && ok; r++) {
+            queued = 0;
+            for (int k = first; k < last && ok; k++) {
+                const int u = vis[k];
+                const int p1 = m.row[u + 1];
+                for (int p = m.row[u]; p < p1 && ok; p += kRingLanes) {
+                    const int x = p + l < p1 ? m.col[p + l] : -1;
+                    bool fresh = absent(vis, nvis, x) && x >= 0;
+                    // a ring lists a vertex once; should it not, its first place counts
+                    const unsigned same = (__match_any_sync(group, x) & group) >> shift;
+                    fresh = fresh && (same & ((1u << l) - 1u)) == 0u;
+                    unsigned add = (__ballot_sync(group, fresh) & group) >> shift;
+                    for (; add && ok; add &= add - 1u)
+                        visit(__shfl_sync(group, x, shift + __ffs((int)add) - 1), queued);
+                }
+            }
+            first = last;
+            last = nvis;
+        }
+        if (l == 0) {
+            if (!ok) atomicAdd(overflow, 1ull);
+            counts[t] = ok ? nf : -1;
+        }
+    }
+    if (l == 0) s_nf[g] = t < n && ok ? nf : 0;
+    __syncthreads();
+    // the block's lists, kRingGroups vertices side by side
+    int most = 0;
+    for (int q = 0; q < kRingGroups; q++) most = max(most, s_nf[q]);
+    const int col = threadIdx.x % kRingGroups;
+    for (int j = threadIdx.x / kRingGroups; j < most; j += kRingLanes)
+        if (j < s_nf[col]) lists[(int64_t)j * n + t0 + col] = s_fl[col][j];
 }
 
 // Inverse of the n x n matrix a by LU decomposition with partial pivoting
 // (Doolittle), one substitution per unit vector; 0 when a pivot is exactly zero.
 template <int N>
 __device__ int curv_lu_invert(const double a[N][N], double ai[N][N]) {
-    double lu[N][N];
+    double lu[N][N], rec[N];
+    bool good[N];
     int piv[N];
     for (int i = 0; i < N; i++)
         for (int j = 0; j < N; j++) lu[i][j] = a[i][j];
@@ -150,8 +316,10 @@ __device__ int curv_lu_invert(const double a[N][N], double ai[N][N]) {
         if (p != k)
             for (int j = 0; j < N; j++) { const double t = lu[k][j]; lu[k][j] = lu[p][j]; lu[p][j] = t; }
         const double d = lu[k][k];
+        good[k] = divides_well(d);
+        rec[k] = 1.0 / d;
         for (int i = k + 1; i < N; i++) {
-            const double f = lu[i][k] / d;
+            const double f = good[k] ? quotient(lu[i][k], d, rec[k]) : lu[i][k] / d;
             lu[i][k] = f;
             for (int j = k + 1; j < N; j++) lu[i][j] -= f * lu[k][j];
         }
@@ -165,7 +333,7 @@ __device__ int curv_lu_invert(const double a[N][N], double ai[N][N]) {
             for (int j = 0; j < i; j++) x[i] -= lu[i][j] * x[j];
         for (int i = N - 1; i >= 0; i--) {
             for (int j = i + 1; j < N; j++) x[i] -= lu[i][j] * x[j];
-            x[i] /= lu[i][i];
+            x[i] = good[i] ? quotient(x[i], lu[i][i], rec[i]) : x[i] / lu[i][i];
         }
         for (int i = 0; i < N; i++) ai[i][c] = x[i];
     }
@@ -214,17 +382,35 @@ __device__ void curv_jacobi2(const double a[2][2], double w[2], double v[2][2]) 
 // vtkSinglePolynomialMeasure::ComputeFitting (Common/vtkCurvatureMeasure.cxx:188-505)
 // on the faces fl[0..nf): returns sqrt(k1^2 + k2^2), info = principal directions
 // scaled by sqrt|k|, the larger |k| first.
-__device__ double curv_fit(const CurvMesh& m, const int* fl, int nf, double* xs, double* ys, double* zs,
+// stride: between the entries of fl.
+__device__ double curv_fit(const CurvMesh& m, const int* fl, int64_t stride, int nf, double* xs, double* ys, double* zs,
                            double info[6]) {
     double sarea = 0, origin[3] = {0, 0, 0}, frame[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    for (int j = 0; j < nf; j++) {
-        const FaceProps& q = m.fp[fl[j]];
-        const double area = q.area;
-        for (int k = 0; k < 3; k++) {
-            origin[k] += area * q.bary[k];
-            frame[0][k] += area * q.n[k];
+    // kFitBatch faces at a time, their records loaded before any is used: the index and the
+    // record it points to are two dependent loads, and a small mesh has few warps to hide them
+    for (int j0 = 0; j0 < nf; j0 += kFitBatch) {
+        int id[kFitBatch];
+        double v[kFitBatch][7];
+#pragma unroll
+        for (int b = 0; b < kFitBatch; b++) id[b] = fl[(j0 + b < nf ? j0 + b : nf - 1) * stride];
+#pragma unroll
+        for (int b = 0; b < kFitBatch; b++) {
+            const FaceProps& q = m.fp[id[b]];
+            for (int k = 0; k < 3; k++) {
+                v[b][k] = q.ab[k];
+                v[b][3 + k] = q.an[k];
+            }
+            v[b][6] = q.area;
         }
-        sarea += area;
+#pragma unroll
+        for (int b = 0; b < kFitBatch; b++) {
+            if (j0 + b >= nf) break;
+            for (int k = 0; k < 3; k++) {
+                origin[k] += v[b][k];
+                frame[0][k] += v[b][3 + k];
+            }
+            sarea += v[b][6];
+        }
     }
     for (int j = 0; j < 3; j++) origin[j] = origin[j] / sarea;
     curv_normalize(frame[0]);
@@ -236,30 +422,56 @@ __device__ double curv_fit(const CurvMesh& m, const int* fl, int nf, double* xs,
     for (int i = 0; i < 6; i++) info[i] = 0;
     if (nf <= 6) return 0;
     double h = 0;
-    for (int j = 0; j < nf; j++) {
-        const FaceProps& fq = m.fp[fl[j]];
-        double bary[3] = {fq.bary[0], fq.bary[1], fq.bary[2]};
-        for (int k = 0; k < 3; k++) bary[k] -= origin[k];
-        const double x = curv_dot(bary, frame[0]), y = curv_dot(bary, frame[1]), z = curv_dot(bary, frame[2]);
-        xs[j] = x; ys[j] = y; zs[j] = z;
-        h += sqrt(x * x + y * y);
+    for (int j0 = 0; j0 < nf; j0 += kFitBatch) {
+        int id[kFitBatch];
+        double c[kFitBatch][3];
+#pragma unroll
+        for (int b = 0; b < kFitBatch; b++) id[b] = fl[(j0 + b < nf ? j0 + b : nf - 1) * stride];
+#pragma unroll
+        for (int b = 0; b < kFitBatch; b++)
+            for (int k = 0; k < 3; k++) c[b][k] = m.fp[id[b]].bary[k];
+#pragma unroll
+        for (int b = 0; b < kFitBatch; b++) {
+            const int j = j0 + b;
+            if (j >= nf) break;
+            double bary[3] = {c[b][0], c[b][1], c[b][2]};
+            for (int k = 0; k < 3; k++) bary[k] -= origin[k];
+            const double x = curv_dot(bary, frame[0]), y = curv_dot(bary, frame[1]), z = curv_dot(bary, frame[2]);
+            xs[j] = x; ys[j] = y; zs[j] = z;
+            h += sqrt(x * x + y * y);
+        }
     }
     h = h / ((double)nf);
-    // normal equations of the conditioned Vandermonde rows (upper half, mirrored)
+    // normal equations of the conditioned Vandermonde rows (upper half, mirrored); the first
+    // entry of a row is 1, and its products are the other factor
     double xxt[6][6], xxti[6][6], xyt[6], q[6];
     for (int i = 0; i < 6; i++) {
         xyt[i] = 0.0;
         for (int j = 0; j < 6; j++) xxt[i][j] = 0.0;
     }
+    const double hh = h * h;
+    const bool good = divides_well(hh) && divides_well(h);
+    const double rh = 1.0 / h, rhh = 1.0 / hh;
     for (int k = 0; k < nf; k++) {
-        const double x = xs[k], y = ys[k];
+        const double x = xs[k], y = ys[k], z = zs[k];
         double r[6] = {1.0, x, y, x * x, x * y, y * y};
-        r[1] /= h; r[2] /= h; r[3] /= h * h; r[4] /= h * h; r[5] /= h * h;
-        for (int i = 0; i < 6; i++) {
+        if (good) {
+            r[1] = quotient(r[1], h, rh); r[2] = quotient(r[2], h, rh);
+            r[3] = quotient(r[3], hh, rhh); r[4] = quotient(r[4], hh, rhh); r[5] = quotient(r[5], hh, rhh);
+        } else {
+            r[1] /= h; r[2] /= h; r[3] /= hh; r[4] /= hh; r[5] /= hh;
+        }
+#pragma unroll
+        for (int j = 1; j < 6; j++) xxt[0][j] += r[j];
+        xyt[0] += z;
+#pragma unroll
+        for (int i = 1; i < 6; i++) {
+#pragma unroll
             for (int j = i; j < 6; j++) xxt[i][j] += r[i] * r[j];
-            xyt[i] += r[i] * zs[k];
+            xyt[i] += r[i] * z;
         }
     }
+    xxt[0][0] = (double)nf;   // nf times 1, exactly
     for (int i = 0; i < 6; i++)
         for (int j = 0; j < i; j++) xxt[i][j] = xxt[j][i];
     if (!curv_lu_invert<6>(xxt, xxti)) return 0;
@@ -288,95 +500,63 @@ __device__ double curv_fit(const CurvMesh& m, const int* fl, int nf, double* xs,
     return sqrt(ev[0] * ev[0] + ev[1] * ev[1]);
 }
 
-// One vertex (original id v): the faces of its 3-ring in the reference's order
-// (vtkNeighbourhoodComputation::ComputeNRingCells, Common/vtkNeighbourhoodComputation.cxx:38-100:
-// the vertex's own faces, then ring by ring the faces of the edges of each vertex
-// not yet visited), then the fit.  A neighbourhood larger than the buffers counts
-// in *overflow and leaves the vertex's outputs at zero.
-__global__ void __launch_bounds__(64) curvature_kernel(CurvMesh m, double* __restrict__ indicator,
-                                                       float* __restrict__ dirs,
-                                                       unsigned long long* __restrict__ overflow) {
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= m.nv) return;
-    int fl[kCurvMaxF];
-    int vis[kCurvMaxVis];
-    int lists[2][kCurvMaxV];
-    int nf = 0, nvis = 0;
-    bool ok = true;
-    auto add_face = [&](int f) {
-        for (int i = 0; i < nf; i++)
-            if (fl[i] == f) return;
-        if (nf < kCurvMaxF) fl[nf++] = f;
-        else ok = false;
-    };
-    {
-        const int t = m.inv[v];
-        for (int p = m.row[t]; p < m.row[t + 1]; p++) {
-            const int e = m.slot_edge[p];
-            if (e < 0) continue;
-            const int2 pf = m.poly[e];
-            if (pf.x >= 0) add_face(pf.x);
-            if (pf.y >= 0) add_face(pf.y);
-        }
-    }
-    int cur = 0, ncur = 1;
-    lists[0][0] = (int)v;
-    for (int r = 0; r < 3 && ok; r++) {
-        int nnext = 0;
-        for (int k = 0; k < ncur && ok; k++) {
-            const int u = lists[cur][k];
-            bool seen = false;
-            for (int i = 0; i < nvis; i++) seen |= vis[i] == u;
-            if (seen) continue;
-            if (nvis == kCurvMaxVis) { ok = false; break; }
-            vis[nvis++] = u;
-            const int tu = m.inv[u];
-            for (int p = m.row[tu]; p < m.row[tu + 1]; p++) {
-                if (nnext == kCurvMaxV) { ok = false; break; }
-                lists[cur ^ 1][nnext++] = m.perm[m.col[p]];
-                const int e = m.slot_edge[p];
-                if (e < 0) continue;
-                const int2 pf = m.poly[e];
-                if (pf.x >= 0) {
-                    add_face(pf.x);
-                    if (pf.y >= 0) add_face(pf.y);
-                }
-            }
-        }
-        cur ^= 1;
-        ncur = nnext;
-    }
+// The fits of vertices v0 .. v0 + n - 1 over their face lists.  A neighbourhood that was too
+// large leaves the vertex's outputs at zero.  One warp per block: the SMs differ by a warp.
+constexpr int kFitThreads = 32;
+
+__global__ void __launch_bounds__(kFitThreads) curvature_kernel(CurvMesh m, int64_t v0, int64_t n,
+                                                                const int* __restrict__ lists,
+                                                                const int* __restrict__ counts,
+                                                                double* __restrict__ indicator,
+                                                                float* __restrict__ dirs) {
+    const int64_t t = (int64_t)blockIdx.x * kFitThreads + threadIdx.x;
+    if (t >= n) return;
+    const int nf = counts[t];
     double info[6] = {0, 0, 0, 0, 0, 0};
     double ind = 0.0;
-    if (ok) {
+    if (nf >= 0) {
         double xs[kCurvMaxF], ys[kCurvMaxF], zs[kCurvMaxF];
-        ind = curv_fit(m, fl, nf, xs, ys, zs, info);
-    } else {
-        atomicAdd(overflow, 1ull);
+        ind = curv_fit(m, lists + t, n, nf, xs, ys, zs, info);
     }
+    const int64_t v = v0 + t;
     indicator[v] = ind;
     for (int i = 0; i < 6; i++) dirs[6 * v + i] = (float)info[i];
 }
 
 static inline unsigned cgrid(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
-size_t curvature_face_bytes(int64_t nf) { return (size_t)nf * sizeof(FaceProps); }
+// Work of launch_curvature: the faces' values, the items' fans and the lists of a chunk.
+static int64_t curv_chunk(int64_t nv) { return nv < kCurvChunk ? nv : kCurvChunk; }
+
+size_t curvature_work_bytes(int64_t nv, int64_t nf, int64_t ne) {
+    return (size_t)nf * sizeof(FaceProps) +
+           sizeof(int) * (size_t)(4 * ne + nv + curv_chunk(nv) * (kCurvMaxF + 1));
+}
 
 cudaError_t launch_curvature(const double* xyz, const int* tri, int64_t nv, int64_t nf, int64_t ne,
                              const int* edge_v, const int* edge_int, const uint32_t* vf_row, const uint32_t* vf_face,
-                             const int* row, const int* col, const int* perm, const int* inv, int2* poly,
-                             int* slot_edge, void* face_work, double* indicator, float* dirs,
-                             unsigned long long* overflow, cudaStream_t s) {
+                             const int* row, const int* col, const int* inv, int2* poly, int* slot_edge, void* work,
+                             double* indicator, float* dirs, unsigned long long* overflow, cudaStream_t s) {
     if (nv == 0) return cudaSuccess;
     cudaError_t err = cudaMemsetAsync(slot_edge, 0xff, 2 * ne * sizeof(int), s);   // -1: no edge
     if (err != cudaSuccess) return err;
     g_launches += 4;
-    FaceProps* fp = (FaceProps*)face_work;
+    FaceProps* fp = (FaceProps*)work;
+    int* fan = (int*)(fp + nf);
+    int* fan_count = fan + 4 * ne;
+    int* counts = fan_count + nv;
+    int* lists = counts + curv_chunk(nv);
     face_props_kernel<<<cgrid(nf, 256), 256, 0, s>>>(xyz, tri, nf, fp);
     edge_faces_kernel<<<cgrid(ne, 256), 256, 0, s>>>(edge_v, ne, tri, vf_row, vf_face, poly);
     slot_edges_kernel<<<cgrid(ne, 256), 256, 0, s>>>(edge_int, ne, row, col, slot_edge);
-    CurvMesh m{xyz, tri, fp, nv, row, col, perm, inv, slot_edge, poly};
-    curvature_kernel<<<cgrid(nv, 64), 64, 0, s>>>(m, indicator, dirs, overflow);
+    fan_kernel<<<cgrid(nv, 256), 256, 0, s>>>(nv, row, slot_edge, poly, fan, fan_count);
+    const CurvMesh m{fp, nv, row, col, inv, fan, fan_count};
+    for (int64_t v0 = 0; v0 < nv; v0 += kCurvChunk) {
+        const int64_t n = nv - v0 < kCurvChunk ? nv - v0 : kCurvChunk;
+        g_launches += 2;
+        ring_faces_kernel<<<cgrid(n, kRingGroups), kRingThreads, 0, s>>>(m, v0, n, lists, counts, overflow);
+        curvature_kernel<<<cgrid(n, kFitThreads), kFitThreads, 0, s>>>(m, v0, n, lists, counts, indicator, dirs);
+    }
     return cudaGetLastError();
 }
 

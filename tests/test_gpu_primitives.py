@@ -12,7 +12,7 @@ from acvd_gb300 import build
 pytestmark = pytest.mark.gpu
 
 HARNESS = r"""
-#include "%s/primitives.cu"
+#include "@SRC@/primitives.cu"
 template <class T> struct Dev {
     T* p = nullptr;
     Dev(const T* h, size_t n) {
@@ -46,6 +46,37 @@ __global__ void roots_kernel(unsigned long long* bad) {
     if (blockIdx.x == 0 && threadIdx.x == 0)
         if (acvd::recip_rn(acvd::root_rn(2.0f)) != __frcp_rn(__fsqrt_rn(2.0f))) atomicAdd(&bad[2], 1ull);
 }
+// quotients by a shared reciprocal against the IEEE division: random significands, exponents
+// within +-60
+__global__ void quotient_kernel(unsigned long long seed, unsigned per, unsigned long long* bad) {
+    unsigned long long x = seed + (unsigned long long)(blockIdx.x * blockDim.x + threadIdx.x) * 0x9e3779b97f4a7c15ull;
+    auto next = [&]() {   // splitmix64 (Steele, Lea, Flood 2014)
+        unsigned long long z = (x += 0x9e3779b97f4a7c15ull);
+        z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+        z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+        return z ^ (z >> 31);
+    };
+    auto number = [&]() {
+        const unsigned long long u = next();
+        const unsigned long long e = 1023ull - 60ull + (next() % 121ull);
+        return __longlong_as_double((long long)((u & 0x800fffffffffffffull) | (e << 52)));
+    };
+    unsigned long long n = 0;
+    for (unsigned i = 0; i < per; i++) {
+        const double b = number(), inv = 1.0 / b;
+        for (int j = 0; j < 8; j++) {
+            const double a = number();
+            n += acvd::quotient(a, b, inv) != a / b;
+        }
+    }
+    if (n) atomicAdd(bad, n);
+}
+extern "C" int test_quotients(unsigned long long seed, unsigned long long* bad) {
+    Dev<unsigned long long> d(bad, 1);
+    quotient_kernel<<<4096, 256>>>(seed, 512, d.p);   // 2^20 threads x 512 divisors x 8
+    cudaMemcpy(bad, d.p, 8, cudaMemcpyDeviceToHost);
+    return (int)cudaDeviceSynchronize();
+}
 extern "C" int test_roots(unsigned long long* bad) {
     Dev<unsigned long long> d(bad, 3);
     roots_kernel<<<2048, 256>>>(d.p);
@@ -59,7 +90,7 @@ extern "C" int test_roots(unsigned long long* bad) {
 def lib(tmp_path_factory):
     d = tmp_path_factory.mktemp("prim")
     src, so = d / "harness.cu", d / "harness.so"
-    src.write_text(HARNESS % build.SRC)
+    src.write_text(HARNESS.replace("@SRC@", build.SRC))
     subprocess.run([build._nvcc(), build.ARCH, "-O3", "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "-o", str(so),
                     str(src), "-lcudart"], check=True, capture_output=True)
     return ctypes.CDLL(str(so))
@@ -87,3 +118,9 @@ def test_short_roots_and_reciprocals_are_correctly_rounded(lib):
     bad = np.zeros(3, dtype=np.uint64)
     assert lib.test_roots(bad.ctypes.data_as(ctypes.c_void_p)) == 0
     np.testing.assert_array_equal(bad, 0)
+
+
+def test_quotients_by_a_shared_reciprocal(lib):
+    bad = np.zeros(1, dtype=np.uint64)
+    assert lib.test_quotients(ctypes.c_ulonglong(12345), bad.ctypes.data_as(ctypes.c_void_p)) == 0
+    assert bad[0] == 0

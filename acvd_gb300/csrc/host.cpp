@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <queue>
 #include <random>
 #include <unordered_map>
@@ -22,12 +23,14 @@ namespace {
 // faces are scanned in order; the pair (v_j, v_j+1) becomes a new edge the first
 // time it is seen; the first two faces using an edge are its Poly1 / Poly2.
 struct EdgeTable {
-    int64_t nv = 0;
-    std::vector<int32_t> v1, v2, poly1, poly2;
+    int64_t nv = 0, ne = 0;
+    std::unique_ptr<int32_t[]> v1, v2, poly1, poly2;         // ne entries
     std::vector<std::pair<int32_t, int32_t>> extra_faces;   // (edge, face) beyond two faces
     std::vector<int64_t> ring_row;                           // ring CSR (edge ids, creation order)
-    std::vector<int32_t> ring_edge;
+    std::unique_ptr<int32_t[]> ring_edge;
 
+    // The lookups are the cost (3 per face): the edges of a lower endpoint lie side by side as
+    // (upper endpoint, edge) pairs, and nothing grows on the way (at most 3 edges per face).
     bool build(int64_t n_vertices, int64_t n_faces, const int32_t* tri) {
         nv = n_vertices;
         // per lower endpoint: list of (upper endpoint, edge id); capacity from a count pass
@@ -36,46 +39,55 @@ struct EdgeTable {
             const int32_t* t = tri + 3 * f;
             if (t[0] == t[1]) continue;
             for (int j = 0; j < 3; j++) {
-                const int32_t a = t[j], b = t[(j + 1) % 3];
+                const int32_t a = t[j], b = t[j == 2 ? 0 : j + 1];
                 if (a < 0 || b < 0 || a >= n_vertices || b >= n_vertices) return false;
                 if (a == b) continue;
                 cap[std::min(a, b) + 1]++;
             }
         }
         for (int64_t v = 0; v < n_vertices; v++) cap[v + 1] += cap[v];
-        std::vector<int32_t> nb_up(cap[n_vertices]), nb_edge(cap[n_vertices]);
+        struct Up {
+            int32_t hi, edge;
+        };
+        const int64_t most = cap[n_vertices];
+        std::unique_ptr<Up[]> up(new Up[most + 1]);
         std::vector<int32_t> fill(n_vertices, 0);
-        v1.clear(); v2.clear(); poly1.clear(); poly2.clear(); extra_faces.clear();
+        v1.reset(new int32_t[most + 1]);
+        v2.reset(new int32_t[most + 1]);
+        poly1.reset(new int32_t[most + 1]);
+        poly2.reset(new int32_t[most + 1]);
+        extra_faces.clear();
+        ring_row.assign(n_vertices + 1, 0);
+        ne = 0;
         for (int64_t f = 0; f < n_faces; f++) {
             const int32_t* t = tri + 3 * f;
             if (t[0] == t[1]) continue;
             for (int j = 0; j < 3; j++) {
-                const int32_t a = t[j], b = t[(j + 1) % 3];
+                const int32_t a = t[j], b = t[j == 2 ? 0 : j + 1];
                 if (a == b) continue;
                 const int32_t lo = std::min(a, b), hi = std::max(a, b);
-                const int64_t base = cap[lo];
-                int32_t e = -1;
-                for (int32_t q = 0; q < fill[lo]; q++)
-                    if (nb_up[base + q] == hi) { e = nb_edge[base + q]; break; }
-                if (e >= 0) {
-                    if (poly1[e] < 0) poly1[e] = (int32_t)f;
-                    else if (poly2[e] >= 0) extra_faces.push_back({e, (int32_t)f});
+                Up* u = up.get() + cap[lo];
+                const int32_t have = fill[lo];
+                int32_t q = 0;
+                while (q < have && u[q].hi != hi) q++;
+                if (q < have) {
+                    const int32_t e = u[q].edge;
+                    if (poly2[e] >= 0) extra_faces.push_back({e, (int32_t)f});
                     else poly2[e] = (int32_t)f;
                     continue;
                 }
-                e = (int32_t)v1.size();
-                v1.push_back(a); v2.push_back(b); poly1.push_back((int32_t)f); poly2.push_back(-1);
-                nb_up[base + fill[lo]] = hi;
-                nb_edge[base + fill[lo]] = e;
-                fill[lo]++;
+                const int32_t e = (int32_t)ne++;
+                v1[e] = a; v2[e] = b; poly1[e] = (int32_t)f; poly2[e] = -1;
+                u[have].hi = hi;
+                u[have].edge = e;
+                fill[lo] = have + 1;
+                ring_row[a + 1]++;
+                ring_row[b + 1]++;
             }
         }
         // rings: edges in creation order (increasing id)
-        ring_row.assign(n_vertices + 1, 0);
-        const int64_t ne = (int64_t)v1.size();
-        for (int64_t e = 0; e < ne; e++) { ring_row[v1[e] + 1]++; ring_row[v2[e] + 1]++; }
         for (int64_t v = 0; v < n_vertices; v++) ring_row[v + 1] += ring_row[v];
-        ring_edge.resize(2 * ne);
+        ring_edge.reset(new int32_t[2 * ne + 1]);
         std::vector<int64_t> pos(ring_row.begin(), ring_row.end() - 1);
         for (int64_t e = 0; e < ne; e++) {
             ring_edge[pos[v1[e]]++] = (int32_t)e;
@@ -120,7 +132,7 @@ int acvd_build_topology(int64_t n_vertices, int64_t n_faces, const int32_t* tri,
     if (n_vertices >= (int64_t)1 << 31) return ACVD_ERR_UNSUPPORTED;
     EdgeTable t;
     if (!t.build(n_vertices, n_faces, tri)) return ACVD_ERR_ARG;
-    const int64_t ne = (int64_t)t.v1.size();
+    const int64_t ne = t.ne;
     if (2 * ne >= (int64_t)1 << 31) return ACVD_ERR_UNSUPPORTED;
     *n_edges = ne;
     if (edge_v)
@@ -145,13 +157,13 @@ int acvd_vertex_weights(int metric, int64_t n_vertices, const double* xyz, int64
     if (!t.build(n_vertices, n_faces, tri)) return ACVD_ERR_ARG;
     std::vector<double> farea(n_faces);
     for (int64_t f = 0; f < n_faces; f++)
-        farea[f] = tri_area(xyz + 3 * tri[3 * f], xyz + 3 * tri[3 * f + 1], xyz + 3 * tri[3 * f + 2]);
+        farea[f] = tri_area(xyz + 3 * tri[3 * f], xyz + 3 * tri[3 * f + 1], xyz + 3 * tri[3 * f + 2]) / 3.0;
     std::vector<int32_t> fl;
     const bool use_ind = indicator && (metric == ACVD_METRIC_QUADRIC_ANISOTROPIC ? gradation != 0.0 : gradation > 0.0);
     for (int64_t v = 0; v < n_vertices; v++) {
         t.vertex_faces(v, fl);
         double a = 0.0;
-        for (int32_t f : fl) a += farea[f] / 3.0;
+        for (int32_t f : fl) a += farea[f];
         double w = a;
         if (use_ind) w = a * std::pow(indicator[v], gradation);
         if (metric == ACVD_METRIC_QUADRIC_ANISOTROPIC) w = (double)(float)w;   // float item weights
@@ -194,14 +206,17 @@ int acvd_initial_sampling_fixed(int64_t n_vertices, const int32_t* csr_row, cons
     for (int64_t i = 0; i < n; i++) items[i] = (int32_t)i;
     std::mt19937 rng;
     rng.seed(0);
-    for (int64_t i = n - 1; i > 0; --i) std::swap(items[i], items[rng() % (uint64_t)n]);
+    // (rng() is a 32-bit number: the 32-bit remainder is the 64-bit one where n fits)
+    const bool small = n <= (int64_t)UINT32_MAX;
+    auto draw = [&]() { return small ? (int64_t)((uint32_t)rng() % (uint32_t)n) : (int64_t)(rng() % (uint64_t)n); };
+    for (int64_t i = n - 1; i > 0; --i) std::swap(items[i], items[draw()]);
     double sw = 0.0;
     for (int64_t i = 0; i < n; i++) sw += weights[i];
     const double target = sw / (double)k;
     int64_t remaining_items = n;
     int32_t remaining = k - offset;
     int64_t first = 0;
-    std::queue<int32_t> q;
+    std::vector<int32_t> q;   // the region's queue: entries before `head` are done
     while (remaining_items > 0 && remaining > 0) {
         bool found = false;
         int32_t item = 0;
@@ -210,18 +225,17 @@ int acvd_initial_sampling_fixed(int64_t n_vertices, const int32_t* csr_row, cons
             if (labels[item] == k) found = true; else first++;
         }
         if (!found) break;
-        while (!q.empty()) q.pop();
-        q.push(item);
+        q.clear();
+        q.push_back(item);
         sw = 0.0;
         remaining--;
-        while (!q.empty()) {
-            item = q.front();
-            q.pop();
+        for (size_t head = 0; head < q.size(); head++) {
+            item = q[head];
             if (labels[item] != k) continue;
             labels[item] = remaining + offset;
             sw += weights[item];
             remaining_items--;
-            for (int32_t p = csr_row[item]; p < csr_row[item + 1]; p++) q.push(csr_col[p]);
+            q.insert(q.end(), csr_col + csr_row[item], csr_col + csr_row[item + 1]);
             if (sw > target) break;
         }
     }
@@ -232,7 +246,7 @@ int acvd_initial_sampling_fixed(int64_t n_vertices, const int32_t* csr_row, cons
         items[i] = (int32_t)i;
         if (labels[i] != k) sizes[labels[i]]++;
     }
-    for (int64_t i = n - 1; i > 0; --i) std::swap(items[i], items[rng() % (uint64_t)n]);
+    for (int64_t i = n - 1; i > 0; --i) std::swap(items[i], items[draw()]);
     first = 0;
     while (remaining) {
         int32_t item = 0;

@@ -164,15 +164,16 @@ def build_topology(n_vertices: int, faces: np.ndarray):
     """Ring CSR (row, col) and edge endpoints in the reference's numbering."""
     lib = load()
     tri = np.ascontiguousarray(faces, dtype=np.int32)
+    # one call into buffers of the largest size (three edges per face; untouched pages cost
+    # nothing), cut to what came
     ne = _i64()
-    _check(lib.acvd_build_topology(n_vertices, tri.shape[0], _ptr(tri), None, None, None, ctypes.byref(ne)),
-           what="acvd_build_topology")
-    row = np.empty(n_vertices + 1, dtype=np.int32)
-    col = np.empty(2 * ne.value, dtype=np.int32)
-    ev = np.empty(2 * ne.value, dtype=np.int32)
+    most = 6 * max(tri.shape[0], 0) + 2
+    row = np.empty(max(n_vertices, 0) + 1, dtype=np.int32)
+    col = np.empty(most, dtype=np.int32)
+    ev = np.empty(most, dtype=np.int32)
     _check(lib.acvd_build_topology(n_vertices, tri.shape[0], _ptr(tri), _ptr(row), _ptr(col), _ptr(ev),
                                    ctypes.byref(ne)), what="acvd_build_topology")
-    return row, col, ev.reshape(-1, 2)
+    return row, col[:2 * ne.value].copy(), ev[:2 * ne.value].copy().reshape(-1, 2)
 
 
 def read_mesh(path: str):

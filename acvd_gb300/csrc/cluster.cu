@@ -1477,18 +1477,25 @@ __global__ void __launch_bounds__(256) fx_maxabs_kernel(DevState st, unsigned* _
     if (threadIdx.x < NA) atomicMax(&maxbits[threadIdx.x], s_mx[threadIdx.x]);
 }
 
-__global__ void begin_sweep_kernel(DevState st, int ncolors, int reset_claims) {
+// The start of a sweep, by one block: the sweep counter, the proposal and work-list counts
+// and this sweep's moves.
+ACVD_DEV void start_sweep(const DevState& st, int ncolors) {
     const int t = threadIdx.x;
-    if (blockIdx.x == 0) {
-        if (t == 0) st.sweep->sweep += 1;
-        if (t < ncolors) st.cand_count[t] = 0u;
-        if (st.work_count)
-            for (int j = t; j < ncolors * kWorkStripes; j += blockDim.x) st.work_count[j] = 0u;
-        if (t < kStripes) st.counters[t * kNumCounters + kCntMoves] = 0ull;   // this sweep's moves
-    }
-    if (reset_claims)
-        for (int64_t k = (int64_t)blockIdx.x * blockDim.x + t; k <= st.k; k += (int64_t)gridDim.x * blockDim.x)
-            st.claim[k] = ~0ull;
+    if (t == 0) st.sweep->sweep += 1;
+    for (int j = t; j < ncolors; j += blockDim.x) st.cand_count[j] = 0u;
+    if (st.work_count)
+        for (int j = t; j < ncolors * kWorkStripes; j += blockDim.x) st.work_count[j] = 0u;
+    for (int j = t; j < kStripes; j += blockDim.x) st.counters[j * kNumCounters + kCntMoves] = 0ull;
+}
+
+ACVD_DEV void reset_claims(const DevState& st) {
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k <= st.k; k += (int64_t)gridDim.x * blockDim.x)
+        st.claim[k] = ~0ull;
+}
+
+__global__ void begin_sweep_kernel(DevState st, int ncolors, int claims) {
+    if (blockIdx.x == 0) start_sweep(st, ncolors);
+    if (claims) reset_claims(st);
 }
 
 // ---------------------------------------------------------------------------
@@ -1678,52 +1685,84 @@ __global__ void __launch_bounds__(256, 2) sweep_run_kernel(SweepRun a) {
 
 // ---------------------------------------------------------------------------
 // Device-side sweep loop: a CUDA-graph WHILE node repeats an IF / ELSE of the
-// relaxed and the exact sweep; these single-thread kernels take, on the device,
+// relaxed and the exact sweep, and the kernel that ends a sweep takes, on the device,
 // the decisions the host loop takes after each sweep (the same ones as block 0 of
 // the persistent kernel), so the sweeps between two convergence events run without
 // returning to the host.
+//
+// One kernel ends a sweep and starts the next (each launch of a graph costs 2-3.5 us here,
+// whatever it does; ending a relaxed sweep with two launches of the energy sum, a copy, a
+// decision and a start kernel took 12 us of 180 at the 1024 x 512 torus): every block
+// resets its part of the claims; a relaxed sweep's blocks each add a chunk of the energies,
+// and the last one to finish adds the chunks (sum_f64's tree, so the same bits), decides
+// and, if the loop goes on, starts the next sweep.
 // ---------------------------------------------------------------------------
-__global__ void loop_start_kernel(const LoopState* ls, const RunFlags* flags, cudaGraphConditionalHandle h_loop,
-                                  cudaGraphConditionalHandle h_mode) {
-    cudaGraphSetConditional(h_loop, 1u);
-    cudaGraphSetConditional(h_mode, (ls->relaxed_ok && !flags->connexity) ? 1u : 0u);
-}
+constexpr int kEndThreads = 256;
+static_assert(kEndThreads == kSumThreads, "a block of sweep_end_kernel adds one chunk of sum_f64");
 
-__global__ void loop_decide_kernel(LoopState* L, const unsigned long long* counters, const double* e_now,
-                                   const RunFlags* flags, int relaxed, cudaGraphConditionalHandle h_loop,
-                                   cudaGraphConditionalHandle h_mode) {
-    long long mods = 0;
-    for (int q = 0; q < kStripes; q++) mods += (long long)counters[q * kNumCounters + kCntMoves];
-    if (relaxed) {
-        const double e = *e_now;
-        if (L->have_prev && !(e < L->e_prev)) L->relaxed_ok = 0;
-        L->e_prev = e;
-        L->have_prev = 1;
-        L->relaxed_run += 1;
+__global__ void __launch_bounds__(kEndThreads) loop_start_kernel(DevState st, LoopState* L, int ncolors,
+                                                                 cudaGraphConditionalHandle h_loop,
+                                                                 cudaGraphConditionalHandle h_mode) {
+    reset_claims(st);
+    if (blockIdx.x != 0) return;
+    start_sweep(st, ncolors);
+    if (threadIdx.x == 0) {
+        L->done = 0u;
+        cudaGraphSetConditional(h_loop, 1u);
+        cudaGraphSetConditional(h_mode, (L->relaxed_ok && !st.flags->connexity) ? 1u : 0u);
     }
-    L->sweeps += 1;
-    L->run += 1;
-    L->moves += mods;
-    L->last_moves = mods;
-    const bool stop = mods == 0 || L->sweeps > L->max_loops || (mods <= L->early / 1000 && L->convergences <= 1);
-    if (stop) L->status = 1;
-    cudaGraphSetConditional(h_loop, stop ? 0u : 1u);
-    cudaGraphSetConditional(h_mode, (L->relaxed_ok && !flags->connexity) ? 1u : 0u);
 }
 
-cudaError_t launch_loop_start(const LoopState* ls, const RunFlags* flags, cudaGraphConditionalHandle h_loop,
-                              cudaGraphConditionalHandle h_mode, cudaStream_t s) {
-    ++g_launches;
-    loop_start_kernel<<<1, 1, 0, s>>>(ls, flags, h_loop, h_mode);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_loop_decide(LoopState* ls, const unsigned long long* counters, const double* e_now,
-                               const RunFlags* flags, bool relaxed, cudaGraphConditionalHandle h_loop,
-                               cudaGraphConditionalHandle h_mode, cudaStream_t s) {
-    ++g_launches;
-    loop_decide_kernel<<<1, 1, 0, s>>>(ls, counters, e_now, flags, relaxed ? 1 : 0, h_loop, h_mode);
-    return cudaGetLastError();
+// partial: a double per chunk of 2,048 clusters (the grid of a relaxed sweep's end), and one more
+template <bool RELAXED>
+__global__ void __launch_bounds__(kEndThreads) sweep_end_kernel(DevState st, LoopState* L, double* partial,
+                                                                int ncolors, cudaGraphConditionalHandle h_loop,
+                                                                cudaGraphConditionalHandle h_mode) {
+    __shared__ int s_last, s_go;
+    reset_claims(st);
+    double e = 0.0;
+    if (RELAXED) {
+        sum_f64_chunk(st.energy, st.k, blockIdx.x, partial);
+        if (threadIdx.x == 0) {
+            __threadfence();
+            s_last = atomicAdd(&L->done, 1u) == gridDim.x - 1u;
+            __threadfence();
+        }
+        __syncthreads();
+        if (!s_last) return;
+        if (gridDim.x > 1) sum_f64_chunk(partial, gridDim.x, 0, partial + gridDim.x);
+        if (threadIdx.x == 0) e = gridDim.x > 1 ? partial[gridDim.x] : partial[0];   // its own write
+    } else if (blockIdx.x != 0) {
+        return;
+    }
+    if (threadIdx.x < 32) {
+        static_assert(kStripes == 32, "a lane per stripe");
+        unsigned long long v = st.counters[threadIdx.x * kNumCounters + kCntMoves];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+        const long long mods = (long long)v;
+        if (threadIdx.x == 0) {
+            if (RELAXED) {
+                if (L->have_prev && !(e < L->e_prev)) L->relaxed_ok = 0;
+                L->e_prev = e;
+                L->have_prev = 1;
+                L->relaxed_run += 1;
+                L->done = 0u;
+            }
+            L->sweeps += 1;
+            L->run += 1;
+            L->moves += mods;
+            L->last_moves = mods;
+            const bool stop =
+                mods == 0 || L->sweeps > L->max_loops || (mods <= L->early / 1000 && L->convergences <= 1);
+            if (stop) L->status = 1;
+            s_go = !stop;
+            cudaGraphSetConditional(h_loop, stop ? 0u : 1u);
+            cudaGraphSetConditional(h_mode, (L->relaxed_ok && !st.flags->connexity) ? 1u : 0u);
+        }
+    }
+    __syncthreads();
+    if (s_go) start_sweep(st, ncolors);
 }
 
 // ---------------------------------------------------------------------------
@@ -2270,11 +2309,35 @@ cudaError_t launch_fx_scale(int metric, const DevState& st, unsigned* maxbits, c
     return cudaGetLastError();
 }
 
-cudaError_t launch_begin_sweep(const DevState& st, int ncolors, bool reset_claims, cudaStream_t s) {
+// blocks that reset the claims of k clusters
+static unsigned claim_grid(int64_t k) { return (unsigned)std::min<int64_t>(nblk(k + 1, kEndThreads), 2 * sm_count()); }
+
+cudaError_t launch_begin_sweep(const DevState& st, int ncolors, bool claims, cudaStream_t s) {
     ++g_launches;
-    // 64 threads per block cover the colour counts and counter stripes in block 0
-    const unsigned grid = reset_claims ? (unsigned)std::min<int64_t>(nblk(st.k + 1, 64), 4 * sm_count()) : 1u;
-    begin_sweep_kernel<<<grid, 64, 0, s>>>(st, ncolors, reset_claims ? 1 : 0);
+    begin_sweep_kernel<<<claims ? claim_grid(st.k) : 1u, kEndThreads, 0, s>>>(st, ncolors, claims ? 1 : 0);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_loop_start(const DevState& st, LoopState* ls, int ncolors, cudaGraphConditionalHandle h_loop,
+                              cudaGraphConditionalHandle h_mode, cudaStream_t s) {
+    ++g_launches;
+    loop_start_kernel<<<claim_grid(st.k), kEndThreads, 0, s>>>(st, ls, ncolors, h_loop, h_mode);
+    return cudaGetLastError();
+}
+
+int64_t sweep_end_partials(int64_t k) {
+    const int64_t per = (int64_t)kSumThreads * kSumPer;
+    return std::max<int64_t>(1, (k + per - 1) / per) + 1;
+}
+
+cudaError_t launch_sweep_end(const DevState& st, LoopState* ls, double* partial, int ncolors, bool relaxed,
+                             cudaGraphConditionalHandle h_loop, cudaGraphConditionalHandle h_mode, cudaStream_t s) {
+    ++g_launches;
+    if (relaxed)
+        sweep_end_kernel<true><<<(unsigned)(sweep_end_partials(st.k) - 1), kEndThreads, 0, s>>>(st, ls, partial, ncolors,
+                                                                                                h_loop, h_mode);
+    else
+        sweep_end_kernel<false><<<claim_grid(st.k), kEndThreads, 0, s>>>(st, ls, partial, ncolors, h_loop, h_mode);
     return cudaGetLastError();
 }
 

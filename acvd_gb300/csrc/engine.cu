@@ -231,9 +231,8 @@ struct acvd_ctx {
     }
     cudaGraphExec_t relaxed_exec = nullptr;
     cudaGraphExec_t loop_exec = nullptr;   // device-side sweep loop (WHILE around relaxed / exact sweep)
-    DBuf<double> loop_energy;              // energy after the loop's last relaxed sweep
-    Scratch loop_scratch;                  // the loop graph's own summation scratch (never shared,
-                                           // so no other call can move it under the graph)
+    DBuf<double> loop_energy;              // the loop graph's own energy partials (never shared, so no
+                                           // other call can move them under the graph)
     void drop_graph() {
         if (sweep_exec) cudaGraphExecDestroy(sweep_exec);
         sweep_exec = nullptr;
@@ -1085,10 +1084,12 @@ extern "C" int acvd_clean_clustering(acvd_ctx* ctx, int32_t* n_disconnected) {
 // one sweep: every colour class once (eval + apply per class).  With kernel
 // timing on, an event pair per colour brackets the evaluation kernel; the pairs
 // are recorded inside the captured graph and read after the sweep's sync.
-static int enqueue_sweep(acvd_ctx* ctx, bool timing, bool relaxed) {
+// start: with the kernel that starts the sweep (the graph loop's sweeps are started by the
+// kernel that ends the one before).
+static int enqueue_sweep(acvd_ctx* ctx, bool timing, bool relaxed, bool start = true) {
     DevState st = ctx->state();
-    CK(launch_begin_sweep(st, ctx->nclasses, !relaxed, ctx->s));   // exact sweeps: claims reset once
-    int64_t kernels = 1;
+    if (start) CK(launch_begin_sweep(st, ctx->nclasses, !relaxed, ctx->s));   // exact sweeps: claims reset once
+    int64_t kernels = start ? 1 : 0;
     for (int c = 0; c < ctx->nclasses; c++) {
         const int item0 = (int)ctx->sweep_off[c];   // classes are contiguous item ranges
         const int64_t cnt = ctx->sweep_off[c + 1] - ctx->sweep_off[c];
@@ -1169,14 +1170,11 @@ static int run_sweep(acvd_ctx* ctx, bool timing, bool relaxed, double* eval_ms, 
 
 // The sweeps between two convergence events as one graph: a kernel sets the loop
 // and mode conditions, then a WHILE node repeats an IF / ELSE whose bodies are the
-// relaxed sweep (+ the energy sum) and the exact sweep, each ending with the
-// decision kernel.  Built once per context (dropped with the sweep graphs).
+// relaxed and the exact sweep, each ending with the kernel that decides and starts
+// the next.  Built once per context (dropped with the sweep graphs).
 static int build_loop_graph(acvd_ctx* ctx) {
     CK(ctx->dls.resize(1));
-    CK(ctx->loop_energy.resize(1));
-    // sizes the loop's summation scratch outside the capture
-    CK(sum_f64(ctx->energy.p, ctx->K, ctx->loop_energy.p, ctx->loop_scratch, ctx->s));
-    CK(cudaStreamSynchronize(ctx->s));
+    CK(ctx->loop_energy.resize(sweep_end_partials(ctx->K)));
     int r = ACVD_OK;
     cudaGraph_t g;
     CK(cudaGraphCreate(&g, 0));
@@ -1192,7 +1190,8 @@ static int build_loop_graph(acvd_ctx* ctx) {
         return code;
     };
     CK(cudaStreamBeginCaptureToGraph(ctx->s, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    if (launch_loop_start(ctx->dls.p, ctx->dflags.p, h_loop, h_mode, ctx->s) != cudaSuccess)
+    const DevState st = ctx->state();
+    if (launch_loop_start(st, ctx->dls.p, ctx->nclasses, h_loop, h_mode, ctx->s) != cudaSuccess)
         return fail_capture(fail(ctx, ACVD_ERR_CUDA, "loop graph: start kernel"));
     cudaGraph_t g2;
     CK(cudaStreamEndCapture(ctx->s, &g2));
@@ -1220,12 +1219,10 @@ static int build_loop_graph(acvd_ctx* ctx) {
         cudaGraph_t bg = ip.conditional.phGraph_out[b];
         const long long k0 = g_launches;
         CK(cudaStreamBeginCaptureToGraph(ctx->s, bg, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-        if ((r = enqueue_sweep(ctx, false, relaxed))) return fail_capture(r);
-        if (relaxed && sum_f64(ctx->energy.p, ctx->K, ctx->loop_energy.p, ctx->loop_scratch, ctx->s) != cudaSuccess)
-            return fail_capture(fail(ctx, ACVD_ERR_CUDA, "loop graph: energy sum"));
-        if (launch_loop_decide(ctx->dls.p, ctx->counters.p, ctx->loop_energy.p, ctx->dflags.p, relaxed, h_loop,
-                               h_mode, ctx->s) != cudaSuccess)
-            return fail_capture(fail(ctx, ACVD_ERR_CUDA, "loop graph: decision kernel"));
+        if ((r = enqueue_sweep(ctx, false, relaxed, false))) return fail_capture(r);
+        if (launch_sweep_end(st, ctx->dls.p, ctx->loop_energy.p, ctx->nclasses, relaxed, h_loop, h_mode, ctx->s) !=
+            cudaSuccess)
+            return fail_capture(fail(ctx, ACVD_ERR_CUDA, "loop graph: end of the sweep"));
         cudaGraph_t bg2;
         CK(cudaStreamEndCapture(ctx->s, &bg2));
         (relaxed ? ctx->loop_relaxed_kernels : ctx->loop_exact_kernels) = g_launches - k0;

@@ -249,6 +249,7 @@ struct LoopState {
     int relaxed_run;          // out: relaxed sweeps run by this launch
     int run;                  // out: sweeps run by this launch
     int status;               // out: 0 running, 1 convergence test met, 2 grid barrier gave up
+    unsigned done;            // blocks of sweep_end_kernel that have added their chunk
 };
 
 // Grid-wide barrier of the persistent kernel (all blocks co-resident: cooperative launch).
@@ -327,13 +328,14 @@ cudaError_t launch_ring8(const int* row, const int* col, int64_t n, int* ring8, 
 cudaError_t launch_begin_sweep(const DevState& st, int ncolors, bool reset_claims, cudaStream_t s);
 // the grid barrier with one block that never arrives (its wait limit's self-check)
 cudaError_t launch_barrier_wait_limit(GridBar* bar, long long max_spins, cudaStream_t s);
-// device-side sweep loop (graph WHILE node): set the loop and mode conditions at the
-// start, and after each sweep (relaxed: e_now holds the energy after the sweep)
-cudaError_t launch_loop_start(const LoopState* ls, const RunFlags* flags, cudaGraphConditionalHandle h_loop,
+// device-side sweep loop (graph WHILE node): the conditions and the first sweep's start, then
+// after each sweep the decisions (relaxed: with the energy) and the next one's start;
+// partial: sweep_end_partials(k) doubles
+int64_t sweep_end_partials(int64_t k);
+cudaError_t launch_loop_start(const DevState& st, LoopState* ls, int ncolors, cudaGraphConditionalHandle h_loop,
                               cudaGraphConditionalHandle h_mode, cudaStream_t s);
-cudaError_t launch_loop_decide(LoopState* ls, const unsigned long long* counters, const double* e_now,
-                               const RunFlags* flags, bool relaxed, cudaGraphConditionalHandle h_loop,
-                               cudaGraphConditionalHandle h_mode, cudaStream_t s);
+cudaError_t launch_sweep_end(const DevState& st, LoopState* ls, double* partial, int ncolors, bool relaxed,
+                             cudaGraphConditionalHandle h_loop, cudaGraphConditionalHandle h_mode, cudaStream_t s);
 cudaError_t launch_relaxed_step(int metric, const DevState& st, int item0, int64_t count, int color, cudaStream_t s);
 cudaError_t launch_fx_scale(int metric, const DevState& st, unsigned* maxbits, cudaStream_t s);
 // blocks: 256-thread blocks per SM (3..5, else the defaults); threads: 128 for

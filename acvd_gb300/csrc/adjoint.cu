@@ -177,7 +177,7 @@ __global__ void adj_cluster(AdjState a, int metric, int level, double thr, bool 
     bool keep[3] = {false, false, false};
     double P[6] = {0, 0, 0, 0, 0, 0};
     if (metric != kIso) {
-        jacobi_eig3<double>(A, lam, V, 64);
+        jacobi_eig3(A, lam, V, 64);
         double aw[3] = {fabs(lam[0]), fabs(lam[1]), fabs(lam[2])};
         const double mx = fmax(aw[0], fmax(aw[1], aw[2]));
         int used = 0;

@@ -117,11 +117,15 @@ ACVD_DEV void load_eval(const DevState& st, int k, EvalRec& e) {
 }
 
 // symmetric 3x3 (compact) times vector
-template <typename T>
-ACVD_DEV void sym_mul(const T a[6], const T v[3], T o[3]) {
+ACVD_DEV void sym_mul(const double a[6], const double v[3], double o[3]) {
     o[0] = a[0] * v[0] + a[1] * v[1] + a[2] * v[2];
     o[1] = a[1] * v[0] + a[3] * v[1] + a[4] * v[2];
     o[2] = a[2] * v[0] + a[4] * v[1] + a[5] * v[2];
+}
+ACVD_DEV void sym_mul(const float a[6], const float v[3], float o[3]) {
+    o[0] = dot3(a[0], v[0], a[1], v[1], a[2], v[2]);
+    o[1] = dot3(a[1], v[0], a[3], v[1], a[4], v[2]);
+    o[2] = dot3(a[4], v[1], a[2], v[0], a[5], v[2]);
 }
 
 // ---------------------------------------------------------------------------
@@ -136,18 +140,21 @@ ACVD_DEV void sym_mul(const T a[6], const T v[3], T o[3]) {
 template <int M>
 ACVD_DEV void modified_cluster(const EvalRec& c, const ItemRec& it, float sgn, int level, float thr,
                                float& Wn, float dm[3], float dn[3]) {
-    Wn = c.W + sgn * it.w;
+    // (a product by sgn = +-1 is exact)
+    Wn = __fadd_rn(c.W, sgn * it.w);
     const float xm[3] = {it.x[0] - c.m[0], it.x[1] - c.m[1], it.x[2] - c.m[2]};
     const float f = sgn * it.w / Wn;
-    dm[0] = f * xm[0]; dm[1] = f * xm[1]; dm[2] = f * xm[2];
+#pragma unroll
+    for (int j = 0; j < 3; j++) dm[j] = __fmul_rn(f, xm[j]);
     float An[6];
 #pragma unroll
-    for (int j = 0; j < 6; j++) An[j] = c.A[j] + sgn * it.A[j];
+    for (int j = 0; j < 6; j++) An[j] = __fadd_rn(c.A[j], sgn * it.A[j]);
     float Aix[3], And[3];
-    sym_mul<float>(it.A, xm, Aix);
-    sym_mul<float>(An, dm, And);
-    const float rn[3] = {c.r[0] + sgn * Aix[0] - And[0], c.r[1] + sgn * Aix[1] - And[1],
-                         c.r[2] + sgn * Aix[2] - And[2]};
+    sym_mul(it.A, xm, Aix);
+    sym_mul(An, dm, And);
+    float rn[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) rn[j] = __fsub_rn(__fadd_rn(c.r[j], sgn * Aix[j]), And[j]);
     pinv_apply<float>(An, rn, dn, level, thr, 8);
 }
 
@@ -155,14 +162,22 @@ ACVD_DEV void modified_cluster(const EvalRec& c, const ItemRec& it, float sgn, i
 // e, ignoring the item's own term: -2 e.g + e^T T e.
 ACVD_DEV float aniso_shift(const EvalRec& c, const float e[3]) {
     float Te[3];
-    sym_mul<float>(c.T, e, Te);
-    return -2.0f * (e[0] * c.g[0] + e[1] * c.g[1] + e[2] * c.g[2]) + (e[0] * Te[0] + e[1] * Te[1] + e[2] * Te[2]);
+    sym_mul(c.T, e, Te);
+    return __fmaf_rn(-2.0f, dot3(e[0], c.g[0], e[1], c.g[1], e[2], c.g[2]),
+                     dot3(e[0], Te[0], e[1], Te[1], e[2], Te[2]));
 }
 
 ACVD_DEV float item_quad(const float T[6], const float v[3]) {
     float Tv[3];
-    sym_mul<float>(T, v, Tv);
-    return v[0] * Tv[0] + v[1] * Tv[1] + v[2] * Tv[2];
+    sym_mul(T, v, Tv);
+    return dot3(v[0], Tv[0], v[1], Tv[1], v[2], Tv[2]);
+}
+
+// The isotropic part of a change, a quotient times a squared distance, and that of the
+// placed vertex added: v + (W' |delta'|^2 - P).
+ACVD_DEV float iso_part(float num, float den, float d2) { return __fmul_rn(__fdiv_rn(num, den), d2); }
+ACVD_DEV float with_placement(float v, float Wn, const float dn[3], float P) {
+    return __fadd_rn(v, __fmaf_rn(Wn, dot3(dn[1], dn[1], dn[0], dn[0], dn[2], dn[2]), -P));
 }
 
 // Removing its anchor item from a QEM cluster breaks the anchor, which the reference
@@ -178,47 +193,48 @@ ACVD_DEV bool is_anchor_item(const EvalRec& eL, int i) {
 template <int M>
 ACVD_DEV float remove_part(const EvalRec& eL, const ItemRec& it, const RunFlags& fl, float cprime[3]) {
     const float xm[3] = {it.x[0] - eL.m[0], it.x[1] - eL.m[1], it.x[2] - eL.m[2]};
-    const float d2 = xm[0] * xm[0] + xm[1] * xm[1] + xm[2] * xm[2];
-    if (M == kIso) return -it.w * eL.W / (eL.W - it.w) * d2;
+    const float d2 = dot3(xm[0], xm[0], xm[1], xm[1], xm[2], xm[2]);
+    if (M == kIso) return iso_part(__fmul_rn(-it.w, eL.W), __fsub_rn(eL.W, it.w), d2);
     if (M == kQEM) {
-        if (eL.anc != 0.0f) return -it.w * d2;   // placed vertex fixed at the anchor: -w |x - p|^2
-        float v = -it.w * eL.W / (eL.W - it.w) * d2;
-        if (fl.constrained && fl.level > 0) {
-            float Wn, dm[3], dn[3];
-            modified_cluster<M>(eL, it, -1.0f, fl.level, fl.thr, Wn, dm, dn);
-            v += Wn * (dn[0] * dn[0] + dn[1] * dn[1] + dn[2] * dn[2]) - eL.P;
-        }
-        return v;
+        if (eL.anc != 0.0f) return __fmul_rn(-it.w, d2);   // placed vertex fixed at the anchor: -w |x - p|^2
+        const float v = iso_part(__fmul_rn(-it.w, eL.W), __fsub_rn(eL.W, it.w), d2);
+        if (!(fl.constrained && fl.level > 0)) return v;
+        float Wn, dm[3], dn[3];
+        modified_cluster<M>(eL, it, -1.0f, fl.level, fl.thr, Wn, dm, dn);
+        return with_placement(v, Wn, dn, eL.P);
     }
     // anisotropic: shift of L's placed vertex, minus the item's own term at L'
-    float Wn, dm[3], dn[3];
+    float Wn, dm[3], dn[3], e[3];
     modified_cluster<M>(eL, it, -1.0f, fl.level, fl.thr, Wn, dm, dn);
-    const float e[3] = {dm[0] + dn[0] - eL.d[0], dm[1] + dn[1] - eL.d[1], dm[2] + dn[2] - eL.d[2]};
-    const float xc[3] = {xm[0] - dm[0] - dn[0], xm[1] - dm[1] - dn[1], xm[2] - dm[2] - dn[2]};
-    cprime[0] = xc[0]; cprime[1] = xc[1]; cprime[2] = xc[2];
-    return aniso_shift(eL, e) - item_quad(it.T, xc);
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        e[j] = __fsub_rn(__fadd_rn(dm[j], dn[j]), eL.d[j]);
+        cprime[j] = __fsub_rn(__fsub_rn(xm[j], dm[j]), dn[j]);
+    }
+    return __fsub_rn(aniso_shift(eL, e), item_quad(it.T, cprime));
 }
 
 template <int M>
 ACVD_DEV float add_part(const EvalRec& eB, const ItemRec& it, const RunFlags& fl) {
     const float xm[3] = {it.x[0] - eB.m[0], it.x[1] - eB.m[1], it.x[2] - eB.m[2]};
-    const float d2 = xm[0] * xm[0] + xm[1] * xm[1] + xm[2] * xm[2];
-    if (M == kIso) return it.w * eB.W / (eB.W + it.w) * d2;
+    const float d2 = dot3(xm[0], xm[0], xm[1], xm[1], xm[2], xm[2]);
+    if (M == kIso) return iso_part(__fmul_rn(it.w, eB.W), __fadd_rn(eB.W, it.w), d2);
     if (M == kQEM) {
-        if (eB.anc != 0.0f) return it.w * d2;
-        float v = it.w * eB.W / (eB.W + it.w) * d2;
-        if (fl.constrained && fl.level > 0) {
-            float Wn, dm[3], dn[3];
-            modified_cluster<M>(eB, it, 1.0f, fl.level, fl.thr, Wn, dm, dn);
-            v += Wn * (dn[0] * dn[0] + dn[1] * dn[1] + dn[2] * dn[2]) - eB.P;
-        }
-        return v;
+        if (eB.anc != 0.0f) return __fmul_rn(it.w, d2);
+        const float v = iso_part(__fmul_rn(it.w, eB.W), __fadd_rn(eB.W, it.w), d2);
+        if (!(fl.constrained && fl.level > 0)) return v;
+        float Wn, dm[3], dn[3];
+        modified_cluster<M>(eB, it, 1.0f, fl.level, fl.thr, Wn, dm, dn);
+        return with_placement(v, Wn, dn, eB.P);
     }
-    float Wn, dm[3], dn[3];
+    float Wn, dm[3], dn[3], e[3], xc[3];
     modified_cluster<M>(eB, it, 1.0f, fl.level, fl.thr, Wn, dm, dn);
-    const float e[3] = {dm[0] + dn[0] - eB.d[0], dm[1] + dn[1] - eB.d[1], dm[2] + dn[2] - eB.d[2]};
-    const float xc[3] = {xm[0] - dm[0] - dn[0], xm[1] - dm[1] - dn[1], xm[2] - dm[2] - dn[2]};
-    return aniso_shift(eB, e) + item_quad(it.T, xc);
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        e[j] = __fsub_rn(__fadd_rn(dm[j], dn[j]), eB.d[j]);
+        xc[j] = __fsub_rn(__fsub_rn(xm[j], dm[j]), dn[j]);
+    }
+    return __fadd_rn(aniso_shift(eB, e), item_quad(it.T, xc));
 }
 
 // ---------------------------------------------------------------------------
@@ -1064,7 +1080,7 @@ ACVD_DEV void update_cluster(const DevState& st, int k, double* cent = nullptr) 
         return;
     }
     double Am[3];
-    sym_mul<double>(A, m, Am);
+    sym_mul(A, m, Am);
     const double r[3] = {b[0] - Am[0], b[1] - Am[1], b[2] - Am[2]};
     double d[3] = {0.0, 0.0, 0.0};
     const bool place = (M == kAniso) || (fl.constrained && fl.level > 0);
@@ -1084,7 +1100,7 @@ ACVD_DEV void update_cluster(const DevState& st, int k, double* cent = nullptr) 
     for (int j = 0; j < 3; j++) u[j] = df_to_d(a[19 + j]);
     const double c[3] = {m[0] + d[0], m[1] + d[1], m[2] + d[2]};
     double Tc[3];
-    sym_mul<double>(T, c, Tc);
+    sym_mul(T, c, Tc);
     const double g[3] = {u[0] - Tc[0], u[1] - Tc[1], u[2] - Tc[2]};
     ev[4] = make_float4((float)A[4], (float)A[5], 0.f, 0.f);
     ev[5] = make_float4((float)T[0], (float)T[1], (float)T[2], (float)T[3]);
@@ -2135,7 +2151,7 @@ __global__ void post_place_kernel(const double* __restrict__ qv, const uint32_t*
     const double P[3] = {start[3 * src], start[3 * src + 1], start[3 * src + 2]};
     const double A[6] = {q[0], q[1], q[2], q[4], q[5], q[7]};
     double AP[3];
-    sym_mul<double>(A, P, AP);
+    sym_mul(A, P, AP);
     const double r[3] = {-q[3] - AP[0], -q[6] - AP[1], -q[8] - AP[2]};
     double d[3];
     pinv_apply<double>(A, r, d, level, 1e-3, 32);

@@ -177,6 +177,18 @@ ACVD_DEV double quotient(double a, double b, double inv) {
     return fma(fma(-b, q, a), inv, q);
 }
 
+// The sums of products of the energy tests, each operation named: with the contraction left
+// to the compiler, the same source gave other last bits in another kernel, and with them
+// other near-tie moves (a persistent sweep kernel parted from the per-phase ones on 3 of
+// 4.26 million moves).
+ACVD_DEV float dot3(float a0, float b0, float a1, float b1, float a2, float b2) {
+    return __fmaf_rn(a2, b2, __fmaf_rn(a0, b0, __fmul_rn(a1, b1)));
+}
+// a b - c d and a b + c d
+ACVD_DEV float diff_prod(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }
+ACVD_DEV float sum_prod(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }
+ACVD_DEV float add_prod(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
 // Tangent and cosine of the Jacobi rotation of cotangent 2 theta: t = sign(theta) /
 // (|theta| + sqrt(theta^2 + 1)), c = 1 / sqrt(t^2 + 1).
 ACVD_DEV void jacobi_rotation(double theta, double& t, double& c) {
@@ -204,14 +216,14 @@ ACVD_DEV void jacobi_rotation(float theta, float& t, float& c) {
 // Golub & Van Loan, Matrix Computations, sec. 8.5).  a = {a00,a01,a02,a11,a12,a22}.
 // On return w holds the eigenvalues and V (columns) the eigenvectors.
 // ---------------------------------------------------------------------------
-template <typename T>
-ACVD_DEV void jacobi_eig3(const T a6[6], T w[3], T V[3][3], int max_sweeps) {
+ACVD_DEV void jacobi_eig3(const double a6[6], double w[3], double V[3][3], int max_sweeps) {
+    using T = double;
     T A[3][3] = {{a6[0], a6[1], a6[2]}, {a6[1], a6[3], a6[4]}, {a6[2], a6[4], a6[5]}};
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
         for (int j = 0; j < 3; j++) V[i][j] = (i == j) ? T(1) : T(0);
-    const T tiny = sizeof(T) == 4 ? T(1e-14) : T(1e-30);
+    const T tiny = T(1e-30);
     for (int s = 0; s < max_sweeps; s++) {
         const T off = A[0][1] * A[0][1] + A[0][2] * A[0][2] + A[1][2] * A[1][2];
         const T dg = A[0][0] * A[0][0] + A[1][1] * A[1][1] + A[2][2] * A[2][2];
@@ -250,6 +262,53 @@ ACVD_DEV void jacobi_eig3(const T a6[6], T w[3], T V[3][3], int max_sweeps) {
     w[0] = A[0][0]; w[1] = A[1][1]; w[2] = A[2][2];
 }
 
+// The float32 form, its operations named.
+ACVD_DEV void jacobi_eig3(const float a6[6], float w[3], float V[3][3], int max_sweeps) {
+    using T = float;
+    T A[3][3] = {{a6[0], a6[1], a6[2]}, {a6[1], a6[3], a6[4]}, {a6[2], a6[4], a6[5]}};
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) V[i][j] = (i == j) ? T(1) : T(0);
+    const T tiny = T(1e-14);
+    for (int s = 0; s < max_sweeps; s++) {
+        const T off = dot3(A[0][1], A[0][1], A[0][2], A[0][2], A[1][2], A[1][2]);
+        const T dg = dot3(A[0][0], A[0][0], A[1][1], A[1][1], A[2][2], A[2][2]);
+        if (!(off > tiny * dg)) break;
+#pragma unroll
+        for (int pq = 0; pq < 3; pq++) {
+            const int p = pq == 2 ? 1 : 0;
+            const int q = pq == 0 ? 1 : 2;
+            const T apq = A[p][q];
+            if (apq == T(0)) continue;
+            const T theta = (A[q][q] - A[p][p]) / (T(2) * apq);
+            T t, c;
+            jacobi_rotation(theta, t, c);
+            const T sn = t * c;
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const T akp = A[k][p], akq = A[k][q];
+                A[k][p] = diff_prod(c, akp, sn, akq);
+                A[k][q] = sum_prod(sn, akp, c, akq);
+            }
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const T apk = A[p][k], aqk = A[q][k];
+                A[p][k] = diff_prod(c, apk, sn, aqk);
+                A[q][k] = sum_prod(sn, apk, c, aqk);
+            }
+            A[p][q] = A[q][p] = T(0);
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const T vkp = V[k][p], vkq = V[k][q];
+                V[k][p] = diff_prod(c, vkp, sn, vkq);
+                V[k][q] = sum_prod(sn, vkp, c, vkq);
+            }
+        }
+    }
+    w[0] = A[0][0]; w[1] = A[1][1]; w[2] = A[2][2];
+}
+
 // Thresholded pseudo-inverse applied to r, as the reference's quadric vertex
 // placement does (Common/vtkQuadricTools.cxx:83-163): eigenvalues are taken in
 // decreasing |lambda|; at most `level` of them, and only those with
@@ -274,7 +333,7 @@ ACVD_DEV void eig_order(EigPair<T>& x, EigPair<T>& y) {
 template <typename T>
 ACVD_DEV int pinv_apply(const T a6[6], const T r[3], T d[3], int level, T thr, int max_sweeps) {
     T w[3], V[3][3];
-    jacobi_eig3<T>(a6, w, V, max_sweeps);
+    jacobi_eig3(a6, w, V, max_sweeps);
     // the eigenpairs in decreasing |lambda|, equal magnitudes in index order (a stable
     // three-element sorting network on registers)
     EigPair<T> e0 = {fabs(w[0]), w[0], V[0][0], V[1][0], V[2][0]};
@@ -289,10 +348,17 @@ ACVD_DEV int pinv_apply(const T a6[6], const T r[3], T d[3], int level, T thr, i
     auto take = [&](const EigPair<T>& e) {
         const bool keep = (mx > T(0)) && (e.a > thr * mx) && (used < level);
         if (keep) {
-            const T proj = (e.v0 * r[0] + e.v1 * r[1] + e.v2 * r[2]) / e.w;
-            d[0] += proj * e.v0;
-            d[1] += proj * e.v1;
-            d[2] += proj * e.v2;
+            if constexpr (sizeof(T) == 4) {
+                const T proj = dot3(e.v0, r[0], e.v1, r[1], e.v2, r[2]) / e.w;
+                d[0] = add_prod(proj, e.v0, d[0]);
+                d[1] = add_prod(proj, e.v1, d[1]);
+                d[2] = add_prod(proj, e.v2, d[2]);
+            } else {
+                const T proj = (e.v0 * r[0] + e.v1 * r[1] + e.v2 * r[2]) / e.w;
+                d[0] += proj * e.v0;
+                d[1] += proj * e.v1;
+                d[2] += proj * e.v2;
+            }
             used++;
         } else {
             rank_def++;

@@ -318,7 +318,16 @@ ACVD_DEV bool ring_connected_pref(const DevState& st, int p0, int p1, int L, con
     return vis == msk;
 }
 
-// One tile of 256 items of a colour class (blockDim.x == 256; every thread of the
+// Items per tile when `blocks` blocks of TB threads share `count` items: whole warps, no more
+// than TB.  An item on a boundary makes about 2.4 energy tasks, which the block's threads
+// share, so a block with TB items runs two rounds of them while other SMs idle.
+template <int TB>
+__host__ __device__ inline int spread_items(int64_t count, int64_t blocks) {
+    const int64_t n = (count + 32 * blocks - 1) / (32 * blocks) * 32;
+    return (int)(n < 32 ? 32 : (n > TB ? TB : n));
+}
+
+// One tile of `per` items of a colour class (blockDim.x == 256; every thread of the
 // block calls it).  Arrays written during a sweep are read through plain
 // pointers: the persistent sweep kernel reads them after other blocks wrote them.
 //
@@ -342,7 +351,7 @@ ACVD_DEV void set_cached_ev(const DevState& st, int i, int4 c, int ev) {
 }
 
 template <int M, int TB = 256>
-ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color, int claims, int64_t tile,
+ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color, int claims, int64_t tile, int per,
                         const int* entries = nullptr, int n_entries = 0) {
     __shared__ int s_idx[TB];                 // work item -> colour-list position
     __shared__ int s_tgt[TB][kMaxTgt];        // work item -> destination clusters (ring order)
@@ -366,8 +375,8 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
     __syncthreads();
     const int epoch = color * kRounds;   // claim epoch of this step's first matching round
     const bool listed = entries != nullptr;
-    const bool in = listed ? (int)threadIdx.x < n_entries : tile * TB + threadIdx.x < count;
-    const int64_t idx_t = listed ? (in ? (int64_t)entries[threadIdx.x] : 0) : tile * TB + threadIdx.x;
+    const bool in = (int)threadIdx.x < (listed ? n_entries : per) && (listed || tile * per + threadIdx.x < count);
+    const int64_t idx_t = listed ? (in ? (int64_t)entries[threadIdx.x] : 0) : tile * per + threadIdx.x;
     const SweepState sw = *st.sweep;
     const RunFlags fl = *st.flags;
     unsigned n_slots = 0, n_bnd = 0, n_tgt = 0, n_cand = 0, n_scr = 0, n_cached = 0;
@@ -741,8 +750,8 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
 // let more of them be in different phases of their tiles.
 template <int M, int B, int TB = 256>
 __global__ void __launch_bounds__(TB, B * 256 / TB) eval_kernel(DevState st, int item0, int64_t count, int color,
-                                                                int claims) {
-    eval_tile<M, TB>(st, item0, count, color, claims, blockIdx.x);
+                                                                int claims, int per) {
+    eval_tile<M, TB>(st, item0, count, color, claims, blockIdx.x, per);
 }
 
 // default blocks per SM: the fused evaluation 4 (isotropic, QEM) and 5 (the
@@ -896,17 +905,21 @@ __global__ void __launch_bounds__(TB, B * 256 / TB) eval_list_kernel(DevState st
     __shared__ unsigned s_cnt[kWorkStripes];
     if (threadIdx.x < kWorkStripes) s_cnt[threadIdx.x] = work_count[color * kWorkStripes + threadIdx.x];
     __syncthreads();
-    unsigned mx = 0;
-    for (int q = 0; q < kWorkStripes; q++) mx = max(mx, s_cnt[q]);
-    const int64_t per = (mx + TB - 1) / TB;   // tiles of the fullest stripe
+    unsigned mx = 0, total = 0;
+    for (int q = 0; q < kWorkStripes; q++) {
+        mx = max(mx, s_cnt[q]);
+        total += s_cnt[q];
+    }
+    const int n = spread_items<TB>(total, gridDim.x);   // entries per tile
+    const int64_t per = (mx + n - 1) / n;               // tiles of the fullest stripe
     const int64_t cap = work_cap(count);
     for (int64_t t = blockIdx.x; t < per * kWorkStripes; t += gridDim.x) {
         const int q = (int)(t % kWorkStripes);
         const int64_t j = t / kWorkStripes;
-        const int64_t have = (int64_t)s_cnt[q] - j * TB;
+        const int64_t have = (int64_t)s_cnt[q] - j * n;
         if (have <= 0) continue;   // block-uniform
-        eval_tile<M, TB>(st, item0, count, color, claims, t, work + q * cap + j * TB,
-                         have < TB ? (int)have : TB);
+        eval_tile<M, TB>(st, item0, count, color, claims, t, n, work + q * cap + j * n,
+                         have < n ? (int)have : n);
     }
 }
 
@@ -1519,12 +1532,8 @@ __global__ void begin_sweep_kernel(DevState st, int ncolors, int claims) {
 // cooperative launch.  Each phase of a sweep (claim reset, evaluation, commit
 // steps, finalisation, energy sum) is a grid-stride pass over the same device
 // functions as the per-phase kernels, in the same order, with a grid barrier
-// between phases.  The float32 energy tests are compiled with FMA contraction, and
-// the compiler contracts them differently inside this kernel than in the per-phase
-// ones: the clusterings agree bit for bit on the test meshes, but on the 4096^2
-// heightfield a few near-tie decisions of the first sweep come out the other way
-// (built with -fmad=false, both schedules give the same clustering there too), and
-// the autotuner's exactness check rejects this schedule.  Block 0
+// between phases.  The operations of the float32 energy tests are named one by one
+// (dot3 and its like), so its clusterings are the per-phase schedule's bit for bit.  Block 0
 // takes the host loop's after-sweep decisions (relaxed -> exact switch, move
 // count, convergence test, sweep cap); the other blocks read them after the
 // sweep's last barrier.
@@ -1596,8 +1605,15 @@ cudaError_t launch_barrier_wait_limit(GridBar* bar, long long max_spins, cudaStr
     return cudaGetLastError();
 }
 
-template <int M>
-__global__ void __launch_bounds__(256, 2) sweep_run_kernel(SweepRun a) {
+// The barrier of a thread-block cluster: every CTA's earlier writes are visible after it.
+ACVD_DEV void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// CLUSTER: the grid is one thread-block cluster and its hardware barrier takes the grid
+// barrier's place (a.bar is not used).  Small meshes run this way: see kClusterCtas.
+template <int M, bool CLUSTER>
+__global__ void __launch_bounds__(256, CLUSTER ? 1 : 2) sweep_run_kernel(SweepRun a) {
     const DevState& st = a.st;
     const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned gstride = gridDim.x * blockDim.x;
@@ -1605,42 +1621,41 @@ __global__ void __launch_bounds__(256, 2) sweep_run_kernel(SweepRun a) {
     volatile LoopState* vls = a.ls;
     extern __shared__ __align__(16) char stage_mem[];   // 8 warps' commit stages
     CommitStage<M>* stage = reinterpret_cast<CommitStage<M>*>(stage_mem);
-    for (;;) {
+    auto barrier = [&]() {
+        if (!CLUSTER) return grid_barrier(a.bar);
+        cluster_barrier();
+        return true;
+    };
+    for (int run = 0;; run++) {
         const bool relaxed = vls->relaxed_ok && !st.flags->connexity;
-        if (lead) {
-            st.sweep->sweep += 1;
-            for (int c = 0; c < a.nclasses; c++) st.cand_count[c] = 0u;
-            for (int q = 0; q < kStripes; q++) st.counters[q * kNumCounters + kCntMoves] = 0ull;
-        }
-        if (!grid_barrier(a.bar)) return;
+        if (blockIdx.x == 0) start_sweep(st, a.nclasses);
+        if (!relaxed) reset_claims(st);   // once per sweep: a taken cluster keeps a marker per step
+        if (!barrier()) return;
         for (int c = 0; c < a.nclasses; c++) {
             const long long o0 = a.off[c];
             const int64_t cnt = a.off[c + 1] - o0;
             if (cnt == 0) continue;
             const int item0 = (int)o0;
-            if (!relaxed) {
-                for (int64_t k = gtid; k <= st.k; k += gstride) st.claim[k] = ~0ull;
-                if (!grid_barrier(a.bar)) return;
-            }
             const unsigned long long t0 = lead ? global_ns() : 0ull;
-            const int64_t ntiles = (cnt + 255) / 256;
+            const int per = spread_items<256>(cnt, gridDim.x);
+            const int64_t ntiles = (cnt + per - 1) / per;
             for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x)
-                eval_tile<M>(st, item0, cnt, c, relaxed ? 0 : 1, t);
-            if (!grid_barrier(a.bar)) return;
+                eval_tile<M>(st, item0, cnt, c, relaxed ? 0 : 1, t, per);
+            if (!barrier()) return;
             if (lead) a.ls->eval_ns += global_ns() - t0;
             if (relaxed) {
                 relaxed_commit_range<M>(st, item0, cnt, c, gtid >> 5, gstride >> 5, stage[threadIdx.x >> 5]);
-                if (!grid_barrier(a.bar)) return;
+                if (!barrier()) return;
                 fx_finalize_range<M>(st, gtid, gstride);
-                if (!grid_barrier(a.bar)) return;
+                if (!barrier()) return;
             } else {
                 apply_range<M>(st, item0, cnt, c, 0, gtid >> 5, gstride >> 5);
-                if (!grid_barrier(a.bar)) return;
+                if (!barrier()) return;
                 for (int r = 1; r < a.match_rounds; r++) {
                     reclaim_range(st, item0, c, r, gtid, gstride);
-                    if (!grid_barrier(a.bar)) return;
+                    if (!barrier()) return;
                     apply_range<M>(st, item0, cnt, c, r, gtid >> 5, gstride >> 5);
-                    if (!grid_barrier(a.bar)) return;
+                    if (!barrier()) return;
                 }
             }
         }
@@ -1653,7 +1668,7 @@ __global__ void __launch_bounds__(256, 2) sweep_run_kernel(SweepRun a) {
             double* pa = a.esum;
             double* pb = a.esum + nb + 1;
             for (int64_t ch = blockIdx.x; ch < nb; ch += gridDim.x) sum_f64_chunk(st.energy, st.k, ch, pa);
-            if (!grid_barrier(a.bar)) return;
+            if (!barrier()) return;
             const double* cur = pa;
             int64_t m = nb;
             double* dst = pb;
@@ -1661,7 +1676,7 @@ __global__ void __launch_bounds__(256, 2) sweep_run_kernel(SweepRun a) {
             while (m > 1) {
                 const int64_t mb = (m + per - 1) / per;
                 for (int64_t ch = blockIdx.x; ch < mb; ch += gridDim.x) sum_f64_chunk(cur, m, ch, dst);
-                if (!grid_barrier(a.bar)) return;
+                if (!barrier()) return;
                 cur = dst;
                 m = mb;
                 double* t = dst;
@@ -1694,8 +1709,8 @@ __global__ void __launch_bounds__(256, 2) sweep_run_kernel(SweepRun a) {
             if (mods == 0 || L->sweeps > L->max_loops || (mods <= L->early / 1000 && L->convergences <= 1))
                 L->status = 1;
         }
-        if (!grid_barrier(a.bar)) return;
-        if (vls->status != 0) return;
+        if (!barrier()) return;
+        if (vls->status != 0 || run + 1 >= a.max_run) return;
     }
 }
 
@@ -2253,7 +2268,8 @@ cudaError_t launch_eval(int metric, const DevState& st, int item0, int64_t count
     if (threads == 128) {
         // 128-thread blocks, as many threads per SM as four blocks of 256
         if (!split) {
-            ACVD_DISPATCH_128(metric, eval_kernel, nblk(count, 128), s, st, item0, count, color, claims ? 1 : 0);
+            const int per = spread_items<128>(count, 8 * sm_count());
+            ACVD_DISPATCH_128(metric, eval_kernel, nblk(count, per), s, st, item0, count, color, claims ? 1 : 0, per);
             return cudaGetLastError();
         }
         const unsigned sgrid =
@@ -2265,8 +2281,10 @@ cudaError_t launch_eval(int metric, const DevState& st, int item0, int64_t count
         return cudaGetLastError();
     }
     if (!split) {
-        ACVD_DISPATCH_B(metric, blocks, default_eval_blocks(metric), eval_kernel, nblk(count), 256, s, st, item0,
-                        count, color, claims ? 1 : 0);
+        const int dflt = default_eval_blocks(metric), b = blocks >= 3 && blocks <= 5 ? blocks : dflt;
+        const int per = spread_items<256>(count, b * sm_count());
+        ACVD_DISPATCH_B(metric, blocks, dflt, eval_kernel, nblk(count, per), 256, s, st, item0, count, color,
+                        claims ? 1 : 0, per);
         return cudaGetLastError();
     }
     const unsigned sgrid = (unsigned)std::min<int64_t>(nblk(count, kScreenTile), sm_count() * screen_blocks_per_sm(metric));
@@ -2357,10 +2375,11 @@ cudaError_t launch_sweep_end(const DevState& st, LoopState* ls, double* partial,
     return cudaGetLastError();
 }
 
+template <bool CLUSTER>
 static const void* sweep_run_fn(int metric) {
-    return metric == kIso ? (const void*)sweep_run_kernel<kIso>
-         : metric == kQEM ? (const void*)sweep_run_kernel<kQEM>
-                          : (const void*)sweep_run_kernel<kAniso>;
+    return metric == kIso ? (const void*)sweep_run_kernel<kIso, CLUSTER>
+         : metric == kQEM ? (const void*)sweep_run_kernel<kQEM, CLUSTER>
+                          : (const void*)sweep_run_kernel<kAniso, CLUSTER>;
 }
 
 static size_t sweep_run_stage_bytes(int metric) {
@@ -2372,7 +2391,7 @@ int sweep_run_blocks_per_sm(int metric) {
     int nb = 0;
     cudaError_t e;
     const int sm = (int)sweep_run_stage_bytes(metric);
-    const void* fn = sweep_run_fn(metric);
+    const void* fn = sweep_run_fn<false>(metric);
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 256, sm);
     return e == cudaSuccess ? nb : 0;
@@ -2382,8 +2401,47 @@ cudaError_t launch_sweep_run(int metric, const SweepRun& a, int grid, cudaStream
     ++g_launches;
     SweepRun arg = a;
     void* args[] = {(void*)&arg};
-    return cudaLaunchCooperativeKernel(sweep_run_fn(metric), dim3((unsigned)grid), dim3(256), args,
+    return cudaLaunchCooperativeKernel(sweep_run_fn<false>(metric), dim3((unsigned)grid), dim3(256), args,
                                        sweep_run_stage_bytes(metric), s);
+}
+
+// One cluster of kClusterCtas CTAs of 256 threads, one to an SM.
+static void cluster_config(int metric, cudaStream_t s, cudaLaunchConfig_t& cfg, cudaLaunchAttribute& at) {
+    at = cudaLaunchAttribute{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kClusterCtas;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg = cudaLaunchConfig_t{};
+    cfg.gridDim = dim3(kClusterCtas);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = sweep_run_stage_bytes(metric);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+}
+
+bool sweep_cluster_available(int metric) {
+    const void* fn = sweep_run_fn<true>(metric);
+    const int sm = (int)sweep_run_stage_bytes(metric);
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at;
+    cluster_config(metric, nullptr, cfg, at);
+    int n = 0;
+    const bool ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) == cudaSuccess &&
+                    cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0;
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+
+cudaError_t launch_sweep_cluster(int metric, const SweepRun& a, cudaStream_t s) {
+    ++g_launches;
+    SweepRun arg = a;
+    void* args[] = {(void*)&arg};
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at;
+    cluster_config(metric, s, cfg, at);
+    return cudaLaunchKernelExC(&cfg, sweep_run_fn<true>(metric), args);
 }
 
 cudaError_t launch_update_all(int metric, const DevState& st, const ClusterOut& out, cudaStream_t s) {

@@ -1277,10 +1277,37 @@ static int sweep_run_grid(acvd_ctx* ctx) {
     return ctx->run_grid;
 }
 
+// Whether the sweeps of the current problem run in one thread-block cluster: the largest
+// colour class holds at most cluster_max items (ACVD_CLUSTER_MAX; 0: never).
+//
+// A mesh of 10,000 vertices has classes of 2,400 items: ten blocks of the evaluation, for
+// which the launches of a colour step (three relaxed, two exact) and the end of the sweep
+// cost more than the work between them.  In a cluster of 16 CTAs the phases are separated by
+// the cluster's hardware barrier instead.  Above, the per-phase kernels' many SMs win.  A
+// converged solve, graph / cluster, in us (tori of these items, K = items / 20; the largest class
+// holds about 24 % of them):
+//   items          2,560        10,240       20,400       40,960
+//   isotropic   2084 / 1873  2240 / 2012  2803 / 2720  3498 / 4033
+//   QEM         3273 / 2879  5545 / 5167  5828 / 6469  6601 / 8989
+//   anisotropic 3995 / 3552  8260 / 7705  7381 / 8264  9124 / 12517
+constexpr int64_t kDefaultClusterMax = 3072;
+
+static bool use_cluster(acvd_ctx* ctx) {
+    if (ctx->has_work) return false;   // split classes asked for (ACVD_SPLIT_MIN): their two kernels
+    int64_t most = 0;
+    for (int c = 0; c < ctx->nclasses; c++) most = std::max(most, ctx->sweep_off[c + 1] - ctx->sweep_off[c]);
+    int64_t limit = kDefaultClusterMax;
+    if (const char* e = std::getenv("ACVD_CLUSTER_MAX")) limit = std::atoll(e);
+    return most <= limit && sweep_cluster_available(ctx->metric);
+}
+
 // Runs colour sweeps on the device until the host loop's convergence test is
-// met (one cooperative launch).  hl carries the loop state in and out.
-static int run_sweeps_persistent(acvd_ctx* ctx, LoopState& hl, acvd_stats& local) {
-    const int grid = sweep_run_grid(ctx);
+// met: one cooperative launch, or (cluster) launches of one cluster, which return after
+// kClusterRun sweeps at most.  hl carries the loop state in and out.
+constexpr int kClusterRun = 4096;
+
+static int run_sweeps_persistent(acvd_ctx* ctx, LoopState& hl, acvd_stats& local, bool cluster) {
+    const int grid = cluster ? kClusterCtas : sweep_run_grid(ctx);
     const int64_t per = 2048;
     const int64_t nb = std::max<int64_t>(1, (ctx->K + per - 1) / per);
     CK(ctx->dls.resize(1));
@@ -1296,7 +1323,7 @@ static int run_sweeps_persistent(acvd_ctx* ctx, LoopState& hl, acvd_stats& local
     hl.last_moves = 0;
     hl.eval_ns = 0;
     CK(cudaMemcpyAsync(ctx->dls.p, &hl, sizeof hl, cudaMemcpyHostToDevice, ctx->s));
-    CK(cudaMemsetAsync(ctx->dbar.p, 0, sizeof(GridBar), ctx->s));
+    if (!cluster) CK(cudaMemsetAsync(ctx->dbar.p, 0, sizeof(GridBar), ctx->s));
     CK(cudaMemcpyAsync(ctx->doff.p, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice, ctx->s));
     SweepRun a;
     a.st = ctx->state();
@@ -1308,6 +1335,18 @@ static int run_sweeps_persistent(acvd_ctx* ctx, LoopState& hl, acvd_stats& local
     a.esum = ctx->esum.p;
     a.log = ctx->slog.p;
     a.log_cap = kSweepLogCap;
+    if (cluster) {
+        a.max_run = kClusterRun;
+        do {
+            CK(launch_sweep_cluster(ctx->metric, a, ctx->s));
+            CK(cudaMemcpyAsync(&hl, ctx->dls.p, sizeof hl, cudaMemcpyDeviceToHost, ctx->s));
+            const int r = sync_counters(ctx);
+            if (r) return r;
+        } while (hl.status == 0);
+        local.relaxed_sweeps += hl.relaxed_run;
+        local.moves += hl.moves;
+        return ACVD_OK;
+    }
     CK(cudaEventRecord(ctx->ev0, ctx->s));
     CK(launch_sweep_run(ctx->metric, a, grid, ctx->s));
     CK(cudaEventRecord(ctx->ev1, ctx->s));
@@ -1446,6 +1485,8 @@ extern "C" int acvd_minimize(acvd_ctx* ctx, acvd_stats* stats) {
         // graph-looped sweeps unless per-sweep events or the per-sweep trace are wanted
         const bool device_loop = !persistent && !timing && !trace && ctx->opts.use_graphs &&
                                  std::getenv("ACVD_HOST_LOOP") == nullptr;
+        // ... by one thread-block cluster where the mesh is small
+        const bool cluster = device_loop && use_cluster(ctx);
         if (slog.f && persistent) {
             status = fail(ctx, ACVD_ERR_UNSUPPORTED, "ACVD_SWEEP_LOG needs the per-phase schedule");
             break;
@@ -1469,7 +1510,7 @@ extern "C" int acvd_minimize(acvd_ctx* ctx, acvd_stats* stats) {
                 hl.relaxed_ok = relaxed_ok ? 1 : 0;
                 hl.have_prev = have_prev ? 1 : 0;
                 hl.e_prev = e_prev;
-                if ((r = run_sweeps_persistent(ctx, hl, local))) { status = r; break; }
+                if ((r = run_sweeps_persistent(ctx, hl, local, false))) { status = r; break; }
                 if (trace) {
                     const int first = sweeps, last = std::min(hl.sweeps, kSweepLogCap);
                     std::vector<SweepLog> lg(std::max(0, last - first));
@@ -1507,7 +1548,8 @@ extern "C" int acvd_minimize(acvd_ctx* ctx, acvd_stats* stats) {
                 hl.relaxed_ok = relaxed_ok ? 1 : 0;
                 hl.have_prev = have_prev ? 1 : 0;
                 hl.e_prev = e_prev;
-                if ((r = run_sweeps_graph(ctx, hl, local))) { status = r; break; }
+                r = cluster ? run_sweeps_persistent(ctx, hl, local, true) : run_sweeps_graph(ctx, hl, local);
+                if (r) { status = r; break; }
                 sweeps = hl.sweeps;
                 relaxed_ok = hl.relaxed_ok != 0;
                 have_prev = hl.have_prev != 0;

@@ -279,7 +279,11 @@ struct SweepRun {
     double* esum;             // energy-sum partials: ceil(K/2048) + ceil(K/2048^2) + 2 doubles
     SweepLog* log;
     int log_cap;
+    int max_run = 1 << 30;    // sweeps after which the kernel returns to the host, its status still 0
 };
+
+// CTAs of the cluster that runs the sweeps of a small mesh (16, the largest cluster there is)
+constexpr int kClusterCtas = 16;
 
 // ---- items / topology (topology.cu) ----
 cudaError_t launch_ring_adjacency(const int* row, const int* col, int64_t n, unsigned* adj, int* max_deg,
@@ -349,6 +353,9 @@ cudaError_t launch_reclaim(const DevState& st, int item0, int64_t count, int col
 // blocks per SM for this metric (0 when the kernel cannot be co-resident).
 int sweep_run_blocks_per_sm(int metric);
 cudaError_t launch_sweep_run(int metric, const SweepRun& a, int grid, cudaStream_t s);
+// the same sweeps by one thread-block cluster
+bool sweep_cluster_available(int metric);
+cudaError_t launch_sweep_cluster(int metric, const SweepRun& a, cudaStream_t s);
 // device outputs of acvd_get_clusters, any may be null: S (3 k), W (k), the compact quadric (9 k)
 // and the FP64 placed vertices (3 k)
 struct ClusterOut {

@@ -77,7 +77,7 @@ class Schedule:
     coloring: str = "jp"           # jp (device Jones-Plassmann) | order | squeeze
     split_min: int | None = None   # None: the engine's threshold; 0: never split
     eval_blocks: int | None = None  # evaluation kernels' blocks per SM (3, 4, 5); None: the defaults
-    eval_threads: int | None = None  # evaluation kernels' threads per block (128); None: 256
+    eval_threads: int | None = None  # evaluation kernels' threads per block; None: 128, or 256 with eval_blocks
     exact: bool = True   # same clustering as the default schedule, bit for bit
 
     def create_env(self) -> dict:

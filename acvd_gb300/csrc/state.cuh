@@ -154,7 +154,9 @@ struct SweepState {
 // and the items one screen block covers; stripe s of a class of `count` items holds
 // its entries at [s * work_cap(count), (s + 1) * work_cap(count)).
 constexpr int kWorkStripes = 16;
-constexpr int kScreenTile = 4096;
+// (2,048: the 900,000-item classes of a 2047 x 1801 grid make 430 tiles for 608 resident
+// blocks; 46.7 ms a solve there, 48.6 with 4,096 and 47.2 with 1,024)
+constexpr int kScreenTile = 2048;
 __host__ __device__ inline int64_t work_cap(int64_t count) {
     const int64_t nb = (count + kScreenTile - 1) / kScreenTile;
     return ((nb + kWorkStripes - 1) / kWorkStripes) * kScreenTile;

@@ -262,51 +262,50 @@ ACVD_DEV void jacobi_eig3(const double a6[6], double w[3], double V[3][3], int m
     w[0] = A[0][0]; w[1] = A[1][1]; w[2] = A[2][2];
 }
 
-// The float32 form, its operations named.
+// The float32 form, its operations named.  The matrix stays symmetric bit for bit (a column's
+// and a row's rotation are the same operations on the same values), so its upper triangle is
+// all that is kept: d = the diagonal, o = (a01, a02, a12).  For the rotation of rows p < q, the
+// third row is r, o[P] = a_pq, o[R] = a_pr and o[Q] = a_qr.
+template <int p, int q, int P, int R, int Q>
+ACVD_DEV void jacobi_step(float d[3], float o[3], float V[3][3]) {
+    const float apq = o[P];
+    if (apq == 0.0f) return;
+    const float theta = (d[q] - d[p]) / (2.0f * apq);
+    float t, c;
+    jacobi_rotation(theta, t, c);
+    const float s = t * c;
+    // columns, then rows, of the 2 x 2 block; its off-diagonal becomes zero
+    const float pp = diff_prod(c, d[p], s, apq), qp = diff_prod(c, apq, s, d[q]);
+    const float pq = sum_prod(s, d[p], c, apq), qq = sum_prod(s, apq, c, d[q]);
+    d[p] = diff_prod(c, pp, s, qp);
+    d[q] = sum_prod(s, pq, c, qq);
+    o[P] = 0.0f;
+    const float rp = o[R], rq = o[Q];
+    o[R] = diff_prod(c, rp, s, rq);
+    o[Q] = sum_prod(s, rp, c, rq);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const float vkp = V[k][p], vkq = V[k][q];
+        V[k][p] = diff_prod(c, vkp, s, vkq);
+        V[k][q] = sum_prod(s, vkp, c, vkq);
+    }
+}
+
 ACVD_DEV void jacobi_eig3(const float a6[6], float w[3], float V[3][3], int max_sweeps) {
-    using T = float;
-    T A[3][3] = {{a6[0], a6[1], a6[2]}, {a6[1], a6[3], a6[4]}, {a6[2], a6[4], a6[5]}};
+    float o[3] = {a6[1], a6[2], a6[4]};
+    w[0] = a6[0]; w[1] = a6[3]; w[2] = a6[5];
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
-        for (int j = 0; j < 3; j++) V[i][j] = (i == j) ? T(1) : T(0);
-    const T tiny = T(1e-14);
+        for (int j = 0; j < 3; j++) V[i][j] = (i == j) ? 1.0f : 0.0f;
     for (int s = 0; s < max_sweeps; s++) {
-        const T off = dot3(A[0][1], A[0][1], A[0][2], A[0][2], A[1][2], A[1][2]);
-        const T dg = dot3(A[0][0], A[0][0], A[1][1], A[1][1], A[2][2], A[2][2]);
-        if (!(off > tiny * dg)) break;
-#pragma unroll
-        for (int pq = 0; pq < 3; pq++) {
-            const int p = pq == 2 ? 1 : 0;
-            const int q = pq == 0 ? 1 : 2;
-            const T apq = A[p][q];
-            if (apq == T(0)) continue;
-            const T theta = (A[q][q] - A[p][p]) / (T(2) * apq);
-            T t, c;
-            jacobi_rotation(theta, t, c);
-            const T sn = t * c;
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const T akp = A[k][p], akq = A[k][q];
-                A[k][p] = diff_prod(c, akp, sn, akq);
-                A[k][q] = sum_prod(sn, akp, c, akq);
-            }
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const T apk = A[p][k], aqk = A[q][k];
-                A[p][k] = diff_prod(c, apk, sn, aqk);
-                A[q][k] = sum_prod(sn, apk, c, aqk);
-            }
-            A[p][q] = A[q][p] = T(0);
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const T vkp = V[k][p], vkq = V[k][q];
-                V[k][p] = diff_prod(c, vkp, sn, vkq);
-                V[k][q] = sum_prod(sn, vkp, c, vkq);
-            }
-        }
+        const float off = dot3(o[0], o[0], o[1], o[1], o[2], o[2]);
+        const float dg = dot3(w[0], w[0], w[1], w[1], w[2], w[2]);
+        if (!(off > 1e-14f * dg)) break;
+        jacobi_step<0, 1, 0, 1, 2>(w, o, V);
+        jacobi_step<0, 2, 1, 0, 2>(w, o, V);
+        jacobi_step<1, 2, 2, 0, 1>(w, o, V);
     }
-    w[0] = A[0][0]; w[1] = A[1][1]; w[2] = A[2][2];
 }
 
 // Thresholded pseudo-inverse applied to r, as the reference's quadric vertex

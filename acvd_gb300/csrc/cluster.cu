@@ -1351,7 +1351,7 @@ template <int M>
 struct CommitStage {
     static constexpr int NA = Layout<M>::acc;
     static constexpr int GROUP = M == kIso ? 4 : (M == kQEM ? 16 : 32);
-    long long v[32][NA];
+    alignas(16) long long v[32][NA];
     int cl[32][2];   // destination and source; -1: none
 };
 
@@ -1435,46 +1435,96 @@ __global__ void __launch_bounds__(kCommitThreads) relaxed_commit_kernel(DevState
                             gridDim.x * kCommitWarps, s[threadIdx.x >> 5]);
 }
 
+// Finalisation: 32 consecutive clusters to a warp.  Their sums lie in one stretch of memory,
+// which the lanes read and write side by side, a component each, by way of shared memory; the
+// record of a cluster is then one lane's work.  (A lane that walked its own cluster's sums
+// touched 32 lines with every load: 19.0 us a launch against 13.6 now on the anisotropic
+// 2047 x 1801 heightfield, 6.4 against 6.2 on the 1024 x 512 quadric torus, where the chain of
+// one record is what is left.)  At least 6 blocks to an SM: the anisotropic record takes 208
+// registers otherwise, and the 2047 x 1801 solve was 1 % slower; at 8 and 10 it spills.
 template <int M>
-ACVD_DEV void fx_finalize_range(const DevState& st, int64_t k0, int64_t kstride) {
-    constexpr int NA = Layout<M>::acc;
-    for (int64_t k = k0; k < st.k; k += kstride) {
-        const int in = st.in_done[k], out = st.out_done[k];
-        st.out_cnt[k] = 0;
-        if (in == 0 && out == 0) continue;
-        st.in_done[k] = 0;
-        st.out_done[k] = 0;
-        st.size[k] += in - out;
-        df* a = st.acc + k * NA;
-        long long* d = st.fx_delta + k * NA;
+ACVD_DEV void fx_finalize_range(const DevState& st, unsigned warp, unsigned nwarps, CommitStage<M>& s) {
+    constexpr int NA = Layout<M>::acc, NE = Layout<M>::ev;
+    const unsigned lane = threadIdx.x & 31u;
+    float2* sums = reinterpret_cast<float2*>(&s.v[0][0]);
+    float4* recs = reinterpret_cast<float4*>(&s.v[0][0]);
+    static_assert(sizeof(s.v) >= 32 * NE * sizeof(float4), "the records take the sums' place");
+    for (int64_t k0 = 32 * (int64_t)warp; k0 < st.k; k0 += 32 * (int64_t)nwarps) {
+        const int64_t k = k0 + lane;
+        int in = 0, out = 0;
+        if (k < st.k) {
+            in = st.in_done[k];
+            out = st.out_done[k];
+            st.out_cnt[k] = 0;
+        }
+        const bool touched = in != 0 || out != 0;
+        const unsigned mask = __ballot_sync(kFull, touched);
+        if (!mask) continue;
+        df* a = st.acc + k0 * NA;
+        long long* d = st.fx_delta + k0 * NA;
         // every load first (independent), then the arithmetic, then the stores
         df al[NA];
         long long dl[NA];
 #pragma unroll
-        for (int q = 0; q < NA; q++) {
-            al[q] = a[q];
-            dl[q] = d[q];
+        for (int t = 0; t < NA; t++) {
+            const unsigned e = lane + 32u * t;
+            al[t] = df_make(0.0f);
+            dl[t] = 0;
+            if (mask >> (e / NA) & 1u) {
+                al[t] = a[e];
+                dl[t] = d[e];
+            }
+        }
+        if (touched) {
+            st.in_done[k] = 0;
+            st.out_done[k] = 0;
+            st.size[k] += in - out;
         }
 #pragma unroll
-        for (int q = 0; q < NA; q++) al[q] = df_add(al[q], from_fixed(dl[q], st.fx_pow[q]));
-        float4 el[Layout<M>::ev];
-        const int ak = anchor_of<M>(st, k);
-        const double e = cluster_record_df<M>(al, *st.flags, el, ak >= 0 ? st.anchor_xyz + 3 * k : nullptr, ak);
-        float4* ev = st.ev + k * Layout<M>::ev;
-#pragma unroll
-        for (int q = 0; q < NA; q++) {
-            a[q] = al[q];
-            d[q] = 0;
+        for (int t = 0; t < NA; t++) {
+            const unsigned e = lane + 32u * t;
+            const df v = df_add(al[t], from_fixed(dl[t], st.fx_pow[e % NA]));
+            sums[e] = make_float2(v.hi, v.lo);
+            if (mask >> (e / NA) & 1u) {
+                a[e] = v;
+                d[e] = 0;
+            }
         }
+        __syncwarp();
+        float4 el[NE];
+        if (touched) {
+            df mine[NA];
 #pragma unroll
-        for (int q = 0; q < Layout<M>::ev; q++) ev[q] = el[q];
-        st.energy[k] = e;
+            for (int q = 0; q < NA; q++) {
+                const float2 v = sums[lane * NA + q];
+                mine[q] = {v.x, v.y};
+            }
+            const int ak = anchor_of<M>(st, k);
+            st.energy[k] = cluster_record_df<M>(mine, *st.flags, el, ak >= 0 ? st.anchor_xyz + 3 * k : nullptr, ak);
+        }
+        __syncwarp();
+        if (touched) {
+#pragma unroll
+            for (int q = 0; q < NE; q++) recs[lane * NE + q] = el[q];
+        }
+        __syncwarp();
+        float4* ev = st.ev + k0 * NE;
+#pragma unroll
+        for (int t = 0; t < NE; t++) {
+            const unsigned e = lane + 32u * t;
+            if (mask >> (e / NE) & 1u) ev[e] = recs[e];
+        }
+        __syncwarp();
     }
 }
 
+constexpr int kFinalizeThreads = 64;   // small blocks: every SM gets some
+
 template <int M>
-__global__ void fx_finalize_kernel(DevState st) {
-    fx_finalize_range<M>(st, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+__global__ void __launch_bounds__(kFinalizeThreads, 6) fx_finalize_kernel(DevState st) {
+    __shared__ CommitStage<M> s[kFinalizeThreads / 32];
+    const unsigned w = threadIdx.x >> 5;
+    fx_finalize_range<M>(st, blockIdx.x * (kFinalizeThreads / 32) + w, gridDim.x * (kFinalizeThreads / 32), s[w]);
 }
 
 // per accumulator component: the largest |contribution| over the items (as float
@@ -1646,7 +1696,9 @@ __global__ void __launch_bounds__(256, CLUSTER ? 1 : 2) sweep_run_kernel(SweepRu
             if (relaxed) {
                 relaxed_commit_range<M>(st, item0, cnt, c, gtid >> 5, gstride >> 5, stage[threadIdx.x >> 5]);
                 if (!barrier()) return;
-                fx_finalize_range<M>(st, gtid, gstride);
+                // neighbouring warps of clusters on different SMs
+                fx_finalize_range<M>(st, (threadIdx.x >> 5) * gridDim.x + blockIdx.x, gstride >> 5,
+                                     stage[threadIdx.x >> 5]);
                 if (!barrier()) return;
             } else {
                 apply_range<M>(st, item0, cnt, c, 0, gtid >> 5, gstride >> 5);
@@ -2333,7 +2385,7 @@ cudaError_t launch_relaxed_step(int metric, const DevState& st, int item0, int64
                                 cudaStream_t s) {
     if (count == 0) return cudaSuccess;
     ACVD_DISPATCH(metric, relaxed_commit_kernel, commit_grid(count), kCommitThreads, s, st, item0, count, color);
-    ACVD_DISPATCH(metric, fx_finalize_kernel, nblk(st.k, 64), 64, s, st);   // small blocks: every SM gets some
+    ACVD_DISPATCH(metric, fx_finalize_kernel, nblk(st.k, kFinalizeThreads), kFinalizeThreads, s, st);
     return cudaGetLastError();
 }
 

@@ -67,6 +67,7 @@ struct acvd_ctx {
     // internal item order: colour classes contiguous (perm: item -> original
     // vertex id, inv: original vertex id -> item); faces and edges in item ids
     DBuf<int> perm, inv, tri_int, edge_int, label_orig;
+    DBuf<uint2> near8;             // which of them are adjacent
     DBuf<int4> ring8;              // first 8 ring slots per item
     // curvature: faces of every edge, edge of every ring slot, per-vertex outputs
     DBuf<int2> curv_poly;
@@ -219,6 +220,7 @@ struct acvd_ctx {
         st.in_done = in_done.p;
         st.out_done = out_done.p;
         st.ring8 = ring8.p;
+        st.near8 = near8.p;
         st.bflag = bflag.p;
         st.tcache = tcache.p;
         st.orig = perm.p;
@@ -618,6 +620,7 @@ int acvd_set_mesh(acvd_ctx* ctx, int64_t n_vertices, const double* xyz, int64_t 
     CK(ctx->col.resize(2 * n_edges));
     CK(ctx->edge_v.resize(2 * n_edges));
     CK(ctx->adj.resize(2 * n_edges));
+    CK(ctx->near8.resize(n_vertices));
     CK(cudaMemcpyAsync(ctx->xyz.p, xyz, 3 * n_vertices * sizeof(double), cudaMemcpyHostToDevice, ctx->s));
     CK(cudaMemcpyAsync(ctx->tri.p, tri, 3 * n_faces * sizeof(int), cudaMemcpyHostToDevice, ctx->s));
     CK(cudaMemcpyAsync(ctx->row.p, csr_row, (n_vertices + 1) * sizeof(int), cudaMemcpyHostToDevice, ctx->s));
@@ -658,7 +661,7 @@ int acvd_set_mesh(acvd_ctx* ctx, int64_t n_vertices, const double* xyz, int64_t 
     CK(ctx->dtmp.resize(2));
     d_maxdeg = (int*)ctx->dtmp.p;
     CK(cudaMemsetAsync(d_maxdeg, 0, sizeof(int), ctx->s));
-    CK(launch_ring_adjacency(ctx->row.p, ctx->col.p, n_vertices, ctx->adj.p, d_maxdeg, ctx->s));
+    CK(launch_ring_adjacency(ctx->row.p, ctx->col.p, n_vertices, ctx->adj.p, ctx->near8.p, d_maxdeg, ctx->s));
     CK(cudaMemcpyAsync(&ctx->max_deg, d_maxdeg, sizeof(int), cudaMemcpyDeviceToHost, ctx->s));
     CK(cudaStreamSynchronize(ctx->s));
     ctx->ready_mesh = true;

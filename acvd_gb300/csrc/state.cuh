@@ -210,6 +210,8 @@ struct DevState {
     // per item, the first 8 ring neighbours (two int4, ring order, -1 padded; slot
     // 7 = -2 when the ring is longer than 8, which then is read from row / col)
     const int4* ring8;
+    // per item with at most 8 neighbours: byte q = the ring slots adjacent to slot q
+    const uint2* near8;
     // internal item order (colour classes contiguous): original vertex id of
     // each item, and the item of each original vertex id
     const int* orig;
@@ -288,7 +290,7 @@ struct SweepRun {
 constexpr int kClusterCtas = 16;
 
 // ---- items / topology (topology.cu) ----
-cudaError_t launch_ring_adjacency(const int* row, const int* col, int64_t n, unsigned* adj, int* max_deg,
+cudaError_t launch_ring_adjacency(const int* row, const int* col, int64_t n, unsigned* adj, uint2* near8, int* max_deg,
                                   cudaStream_t s);
 cudaError_t launch_color_round(const int* row, const int* col, int64_t n, int* color,
                                unsigned long long* remaining, int* max_color, cudaStream_t s);

@@ -15,7 +15,8 @@ namespace acvd {
 // connectivity constraint is on.
 // ---------------------------------------------------------------------------
 __global__ void ring_adjacency_kernel(const int* __restrict__ row, const int* __restrict__ col, int64_t n,
-                                      unsigned* __restrict__ adj, int* __restrict__ max_deg) {
+                                      unsigned* __restrict__ adj, uint2* __restrict__ near8,
+                                      int* __restrict__ max_deg) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int d_or = i < n ? row[i + 1] - row[i] : 0;
     const int dmax = __reduce_max_sync(kFull, d_or);   // one atomic per warp
@@ -27,6 +28,7 @@ __global__ void ring_adjacency_kernel(const int* __restrict__ row, const int* __
         for (int p = p0; p < p1; p++) adj[p] = 0u;
         return;
     }
+    uint2 near = make_uint2(0u, 0u);
     for (int p = 0; p < d; p++) {
         const int u = col[p0 + p];
         const int u0 = row[u], u1 = row[u + 1];
@@ -37,14 +39,17 @@ __global__ void ring_adjacency_kernel(const int* __restrict__ row, const int* __
                 if (q != p && col[p0 + q] == w) m |= 1u << q;
         }
         adj[p0 + p] = m;
+        if (p < 4) near.x |= (m & 255u) << (8 * p);
+        else if (p < 8) near.y |= (m & 255u) << (8 * (p - 4));
     }
+    near8[i] = near;
 }
 
-cudaError_t launch_ring_adjacency(const int* row, const int* col, int64_t n, unsigned* adj, int* max_deg,
+cudaError_t launch_ring_adjacency(const int* row, const int* col, int64_t n, unsigned* adj, uint2* near8, int* max_deg,
                                   cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     ++g_launches;
-    ring_adjacency_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(row, col, n, adj, max_deg);
+    ring_adjacency_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(row, col, n, adj, near8, max_deg);
     return cudaGetLastError();
 }
 

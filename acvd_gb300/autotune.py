@@ -21,7 +21,7 @@ Two families of candidates:
       blocks of 256 threads per SM (80, 64 or 48 registers per thread) instead of the
       per-kernel defaults;
     - ``threads128``: the evaluation kernels in blocks of 128 threads (8 per SM, 64
-      registers): a block waits at its tile's barriers, and smaller blocks let more of them
+      registers; the default shape): a block waits at its tile's barriers, and smaller blocks let more of them
       be in different phases.
   A candidate of this family whose labels differ from the default's is rejected, since that
   would mean a broken guarantee rather than a faster schedule.

@@ -1,8 +1,7 @@
 // Clustering kernels: the deterministic parallel form of the reference's
 // boundary-swap loop (Common/vtkUniformClustering.h:833-995), the per-cluster
 // statistics (ReComputeStatistics :376-403), connectivity cleaning
-// (CleanClustering :406-549), hole filling (FillHolesInClustering :552-633) and
-// the dual mesh (DiscreteRemeshing/vtkDiscreteRemeshing.h:1003-1152).
+// (CleanClustering :406-549) and hole filling (FillHolesInClustering :552-633).
 //
 // Schedule: the items are coloured once (no two adjacent items share a colour).
 // One step handles one colour class: `eval` proposes, for every boundary item of
@@ -356,7 +355,14 @@ __host__ __device__ inline int spread_items(int64_t count, int64_t blocks) {
     return (int)(n < 32 ? 32 : (n > TB ? TB : n));
 }
 
-// One tile of `per` items of a colour class (blockDim.x == 256; every thread of the
+// A new evaluation sweep for an item whose screen record c is valid (bflag 2): into
+// the record, or, beyond the sweeps a record holds, the item is screened in full next.
+ACVD_DEV void set_cached_ev(const DevState& st, int i, int4 c, int ev) {
+    if (ev < kCacheSweeps) st.tcache[i] = screen_with_ev(c, ev);
+    else st.bflag[i] = 1;
+}
+
+// One tile of `per` items of a colour class (blockDim.x == TB; every thread of the
 // block calls it).  Arrays written during a sweep are read through plain
 // pointers: the persistent sweep kernel reads them after other blocks wrote them.
 //
@@ -372,13 +378,6 @@ __host__ __device__ inline int spread_items(int64_t count, int64_t blocks) {
 // List mode (entries != nullptr): the tile's items are entries[0 .. n_entries), the
 // colour-list positions a screen_kernel pass forwarded (see below); they were
 // counted as visited there.
-// A new evaluation sweep for an item whose screen record c is valid (bflag 2): into
-// the record, or, beyond the sweeps a record holds, the item is screened in full next.
-ACVD_DEV void set_cached_ev(const DevState& st, int i, int4 c, int ev) {
-    if (ev < kCacheSweeps) st.tcache[i] = screen_with_ev(c, ev);
-    else st.bflag[i] = 1;
-}
-
 template <int M, int TB = 256>
 ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color, int claims, int64_t tile, int per,
                         const int* entries = nullptr, int n_entries = 0) {

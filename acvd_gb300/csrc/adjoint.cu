@@ -19,7 +19,7 @@
 // one divisor take one division, and the records that a gather reads are 16-byte aligned.
 // At 512 x 512, K = 10,000, density exponent 1: the two face passes 441 -> 114 us (backward)
 // and 52 -> 39 us, the vertex passes 91 -> 28, the cluster sums 68 -> 35 and the clusters'
-// decompositions 62 -> 42-55 us; forward and backward together 1.25 -> 0.63 ms.
+// decompositions 62 -> 30-43 us; forward and backward together 1.25 -> 0.62 ms.
 #include <cmath>
 
 #include "common.cuh"
@@ -151,6 +151,63 @@ ACVD_DEV void smul(const double a[6], const double v[3], double o[3]) {
     o[2] = a[2] * v[0] + a[4] * v[1] + a[5] * v[2];
 }
 
+// Eigenvalues and eigenvectors (columns of V) of the symmetric a = {a00, a01, a02, a11, a12,
+// a22} by cyclic Jacobi rotations (Golub & Van Loan, Matrix Computations, sec. 8.5), the upper
+// triangle only: w = the diagonal, o = (a01, a02, a12).  The rotation of rows p < q, the third
+// row r (o[P] = a_pq, o[R] = a_pr, o[Q] = a_qr), from two reciprocal roots: with
+// x = a_qq - a_pp, y = 2 a_pq and h = 1 / |(x, y)|, cos^2 = (1 + |x| h) / 2, sin = |y| h / 2 / cos.
+// A cluster's decomposition is one chain of dependent FP64 operations, and there are about 2
+// warps of clusters to an SM, so what counts is the chain: about 30 operations a rotation;
+// with tangent and cosine by three quotients and two roots it was about 55.
+// A decomposition's residual and the columns' deviation from orthonormal are half of what they
+// were (on random sums of 60 normals: 1e-16 and 1.4e-16 root mean square).  At K = 10,000:
+// adj_cluster 42 -> 30 us forward, 55 -> 43 with the backward.  a is a sum of n n^T of unit
+// normals: no entry's square overflows.
+template <int p, int q, int P, int R, int Q>
+ACVD_DEV void adj_rotate(double w[3], double o[3], double V[3][3]) {
+    const double x = w[q] - w[p], y = 2.0 * o[P];
+    const double r2 = x * x + y * y;
+    if (o[P] == 0.0 || !(r2 > 1e-290)) return;
+    const double h = rsqrt(r2);
+    const double c2 = 0.5 + 0.5 * (fabs(x) * h);
+    const double ic = rsqrt(c2);
+    const double sy = 0.5 * (x >= 0.0 ? y : -y) * h;
+    double c = c2 * ic, s = sy * ic;
+    const double e = 0.5 * fma(-c, c, fma(-s, s, 1.0));   // cos^2 + sin^2 = 1 to the last place
+    c += c * e;
+    s += s * e;
+    const double t = s * ic;
+    w[p] -= t * o[P];
+    w[q] += t * o[P];
+    o[P] = 0.0;
+    const double rp = o[R], rq = o[Q];
+    o[R] = c * rp - s * rq;
+    o[Q] = s * rp + c * rq;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const double vkp = V[k][p], vkq = V[k][q];
+        V[k][p] = c * vkp - s * vkq;
+        V[k][q] = s * vkp + c * vkq;
+    }
+}
+
+ACVD_DEV void adj_eig3(const double a[6], double w[3], double V[3][3]) {
+    double o[3] = {a[1], a[2], a[4]};
+    w[0] = a[0]; w[1] = a[3]; w[2] = a[5];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) V[i][j] = i == j ? 1.0 : 0.0;
+    for (int it = 0; it < 64; it++) {
+        const double off = o[0] * o[0] + o[1] * o[1] + o[2] * o[2];
+        const double dg = w[0] * w[0] + w[1] * w[1] + w[2] * w[2];
+        if (!(off > 1e-30 * dg)) break;
+        adj_rotate<0, 1, 0, 1, 2>(w, o, V);
+        adj_rotate<0, 2, 1, 0, 2>(w, o, V);
+        adj_rotate<1, 2, 2, 0, 1>(w, o, V);
+    }
+}
+
 // per cluster: placement, energy, and (bwd) the cotangents of S, W, A, b
 // gE: the cotangent of the total energy, read from dgE (device) when that is given
 __global__ void adj_cluster(AdjState a, int metric, int level, double thr, bool bwd, double gE_host,
@@ -177,7 +234,7 @@ __global__ void adj_cluster(AdjState a, int metric, int level, double thr, bool 
     bool keep[3] = {false, false, false};
     double P[6] = {0, 0, 0, 0, 0, 0};
     if (metric != kIso) {
-        jacobi_eig3(A, lam, V, 64);
+        adj_eig3(A, lam, V);
         double aw[3] = {fabs(lam[0]), fabs(lam[1]), fabs(lam[2])};
         const double mx = fmax(aw[0], fmax(aw[1], aw[2]));
         int used = 0;

@@ -15,7 +15,7 @@
 // run too (79 % busy in the points kernel, 51 us), and the partial stores of 24- and 48-byte
 // strides with a thread per point or face.  So a value is rounded to float on its bits, one
 // FP64 addition per midpoint coordinate is left, and a warp writes its points and faces
-// element by element through shared memory: 95.6 us a level before, 64.4 so.  No access
+// element by element through shared memory: 95.6 us a level before, 62.6 so.  No access
 // is wider than its elements, so the caller's buffers need no alignment beyond theirs.
 // (A thread per output coordinate, and four lanes per face for its three ring searches, were
 // slower: 128 us.)
@@ -31,6 +31,12 @@ constexpr int kSubWarps = kSubThreads / 32;
 
 inline unsigned sgrid(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
+// The rare cases of the two functions below are calls, so that they are branched around:
+// inlined, the compiler ran their FP64 operations for every value and picked the result
+// (FP64 pipe 44 % busy in the points kernel, 64.4 us a level against 62.6).
+__device__ __noinline__ double float_rounded_rare(double v) { return (double)__double2float_rn(v); }
+__device__ __noinline__ double half_rare(double v) { return 0.5 * v; }
+
 // (double)(float)v, rounded to nearest even on the bits where the result is a normal float
 __device__ __forceinline__ double float_rounded(double v) {
     const long long u = __double_as_longlong(v);
@@ -40,7 +46,7 @@ __device__ __forceinline__ double float_rounded(double v) {
         return __longlong_as_double(r);
     }
     if ((u << 1) == 0) return v;   // zeros
-    return (double)__double2float_rn(v);
+    return float_rounded_rare(v);
 }
 
 // v / 2 on the exponent
@@ -48,7 +54,7 @@ __device__ __forceinline__ double half_of(double v) {
     const long long u = __double_as_longlong(v);
     const unsigned e = (unsigned)(u >> 52) & 0x7ffu;
     if (e - 2u < 2045u) return __longlong_as_double(u - (1ll << 52));
-    return 0.5 * v;
+    return (u << 1) == 0 ? v : half_rare(v);
 }
 
 // The slot of b in a's ring, -1 if it is not there.  Four slots are loaded at a time: one by

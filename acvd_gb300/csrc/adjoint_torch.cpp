@@ -51,8 +51,11 @@ const double* dptr(const Tensor& t) { return t.defined() ? t.data_ptr<double>() 
 double* dptr_mut(Tensor& t) { return t.defined() ? t.data_ptr<double>() : nullptr; }
 
 struct ClusteringEnergy : public torch::autograd::Function<ClusteringEnergy> {
-    static variable_list forward(AutogradContext* actx, Tensor xyz, Tensor rho, int64_t engine, double gradation,
-                                 int64_t k) {
+    // (an undefined tensor is no input of a Function: its record of the inputs asks each for
+    // its device, so the densities are optional here too)
+    static variable_list forward(AutogradContext* actx, Tensor xyz, c10::optional<Tensor> density, int64_t engine,
+                                 double gradation, int64_t k) {
+        const Tensor rho = density.has_value() ? *density : Tensor();
         TORCH_CHECK(xyz.is_cuda() && xyz.dim() == 2 && xyz.size(1) == 3, "xyz must be a CUDA (N, 3) tensor");
         TORCH_CHECK(!rho.defined() || (rho.is_cuda() && rho.numel() == xyz.size(0)), "rho must be a CUDA (N,) tensor");
         const c10::cuda::CUDAGuard guard(xyz.device());
@@ -97,7 +100,7 @@ struct ClusteringEnergy : public torch::autograd::Function<ClusteringEnergy> {
 // (energy, centroids) of the engine's fixed clustering; engine = the acvd_ctx pointer
 std::vector<Tensor> clustering_energy(Tensor xyz, c10::optional<Tensor> rho, int64_t engine, double gradation,
                                       int64_t k) {
-    return ClusteringEnergy::apply(xyz, rho.has_value() ? *rho : Tensor(), engine, gradation, k);
+    return ClusteringEnergy::apply(xyz, rho, engine, gradation, k);
 }
 
 }  // namespace

@@ -327,15 +327,18 @@ class Engine:
         return int(self._lib.acvd_stream(self.ctx) or 0)
 
     def set_mesh(self, points, faces, row, col, edge_v):
-        self._pts = np.ascontiguousarray(points, dtype=np.float64)
-        self._tri = np.ascontiguousarray(faces, dtype=np.int32)
+        pts = np.ascontiguousarray(points, dtype=np.float64)
+        tri = np.ascontiguousarray(faces, dtype=np.int32)
         row = np.ascontiguousarray(row, dtype=np.int32)
         col = np.ascontiguousarray(col, dtype=np.int32)
         ev = np.ascontiguousarray(edge_v, dtype=np.int32)
-        self.n = self._pts.shape[0]
+        self._ck(self._lib.acvd_set_mesh(self.ctx, pts.shape[0], _ptr(pts), tri.shape[0], _ptr(tri),
+                                         _ptr(row), _ptr(col), ev.size // 2, _ptr(ev)), "acvd_set_mesh")
+        # only now: a refused mesh leaves the context the one it holds, whose sizes the
+        # buffers of its outputs need
+        self._pts, self._tri = pts, tri
+        self.n = pts.shape[0]
         self.n_edges = ev.size // 2
-        self._ck(self._lib.acvd_set_mesh(self.ctx, self.n, _ptr(self._pts), self._tri.shape[0], _ptr(self._tri),
-                                         _ptr(row), _ptr(col), self.n_edges, _ptr(ev)), "acvd_set_mesh")
 
     def set_metric(self, metric: str, indicator=None, principal_dirs=None, gradation: float = 0.0):
         ind = None if indicator is None else np.ascontiguousarray(indicator, dtype=np.float64)

@@ -376,8 +376,10 @@ class Engine:
 
     def set_labels(self, k: int, labels):
         lab = np.ascontiguousarray(labels, dtype=np.int32)
-        self.k = int(k)
-        self._ck(self._lib.acvd_set_labels(self.ctx, self.k, _ptr(lab)), "acvd_set_labels")
+        k = int(k)
+        if 0 < k < 1 << 21:   # others are refused at once: the context keeps its clusters
+            self.k = k
+        self._ck(self._lib.acvd_set_labels(self.ctx, k, _ptr(lab)), "acvd_set_labels")
 
     def rewind(self):
         self._ck(self._lib.acvd_rewind(self.ctx), "acvd_rewind")

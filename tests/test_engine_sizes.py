@@ -1,6 +1,6 @@
-"""Buffers of the outputs after a refused mesh (CPU; the library is a stand-in): the context
-keeps its mesh when acvd_set_mesh refuses its arguments, so the outputs still have that
-mesh's sizes.
+"""Buffers of the outputs after a refused mesh or cluster count (CPU; the library is a
+stand-in): the context keeps what it holds when acvd_set_mesh or acvd_set_labels refuses its
+arguments, so the outputs still have those sizes.
 """
 import ctypes
 
@@ -20,6 +20,12 @@ class _Lib:
         self.n, self.nf, self.ne = n, nf, ne
         return 0
 
+    def acvd_set_labels(self, ctx, k, lab):
+        if k <= 0 or k >= 1 << 21:
+            return 1 if k <= 0 else 3
+        self.k = k
+        return 0
+
     def acvd_last_error(self, ctx):
         return b"refused"
 
@@ -35,6 +41,10 @@ class _Lib:
     def acvd_get_dual_mesh(self, ctx, out, n):
         self.room = 3 * self.nf
         n._obj.value = 0
+        return 0
+
+    def acvd_get_clusters(self, ctx, *a):
+        self.room = self.k
         return 0
 
     def acvd_destroy(self, ctx):
@@ -85,3 +95,14 @@ def test_outputs_keep_the_mesh_that_is_held(engine, what, output):
     engine.sizes.clear()
     getattr(engine, output)()
     assert engine.sizes[0] >= engine._lib.room
+
+
+@pytest.mark.parametrize("k", [0, -3, 1 << 21])
+def test_outputs_keep_the_clusters_that_are_held(engine, k):
+    engine.set_mesh(*_mesh(50))
+    engine.set_labels(7, np.zeros(52, dtype=np.int32))
+    with pytest.raises(AcvdError):
+        engine.set_labels(k, np.zeros(52, dtype=np.int32))
+    engine.sizes.clear()
+    engine.clusters()
+    assert engine.sizes[0] == engine._lib.room == engine.k

@@ -168,7 +168,10 @@ __global__ void face_props_kernel(const double* __restrict__ xyz, const int* __r
 }
 
 // The faces around item i in the order its ring's edges name them (each edge's first two
-// faces), each once: the order in which vtkNeighbourhoodComputation meets them.
+// faces), each once: the order in which vtkNeighbourhoodComputation meets them.  More than
+// kCurvMaxF faces are past the bound of every ring that holds the item, so that the list stops
+// there: each face is looked up among those before it, and a hub of 60,000 would take this
+// one thread 10^9 dependent loads.
 __global__ void fan_kernel(int64_t n, const int* __restrict__ row, const int* __restrict__ slot_edge,
                            const int2* __restrict__ poly, int* fan, int* __restrict__ fan_count) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -181,7 +184,7 @@ __global__ void fan_kernel(int64_t n, const int* __restrict__ row, const int* __
             if (out[j] == f) return;
         out[c++] = f;
     };
-    for (int p = p0; p < p1; p++) {
+    for (int p = p0; p < p1 && c <= kCurvMaxF; p++) {
         const int e = slot_edge[p];
         if (e < 0) continue;
         const int2 pf = poly[e];

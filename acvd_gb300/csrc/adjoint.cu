@@ -51,10 +51,13 @@ __global__ void adj_face_fwd(AdjState a) {
     const double cr[3] = {e1[1] * e2[2] - e1[2] * e2[1], e1[2] * e2[0] - e1[0] * e2[2], e1[0] * e2[1] - e1[1] * e2[0]};
     const double L = sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
     double n[3] = {0.0, 0.0, 0.0};
-    if (L > 1e-300) {
+    QuotientRange range;
+    range.add(L);
+    for (int d = 0; d < 3; d++) range.add(cr[d]);
+    if (L > 0.0 && range.holds()) {
         const double inv = 1.0 / L;
-        for (int d = 0; d < 3; d++) n[d] = quotient(cr[d], L, inv);
-    } else if (L > 0.0) {   // 1 / L may overflow
+        for (int d = 0; d < 3; d++) n[d] = quotient_in_range(cr[d], L, inv);
+    } else if (L > 0.0) {
         for (int d = 0; d < 3; d++) n[d] = cr[d] / L;
     }
     put2(a.face + 4 * f, n[0], n[1]);
@@ -398,10 +401,13 @@ __global__ void adj_face_bwd(AdjState a) {
     if (L > 0.0) {
         const double ngn = n[0] * g_n[0] + n[1] * g_n[1] + n[2] * g_n[2];
         double h[3] = {g_n[0] - n[0] * ngn, g_n[1] - n[1] * ngn, g_n[2] - n[2] * ngn};
-        if (L > 1e-300) {
+        QuotientRange range;
+        range.add(L);
+        for (int d = 0; d < 3; d++) range.add(h[d]);
+        if (range.holds()) {
             const double inv = 1.0 / L;
-            for (int d = 0; d < 3; d++) h[d] = quotient(h[d], L, inv);
-        } else {   // 1 / L may overflow
+            for (int d = 0; d < 3; d++) h[d] = quotient_in_range(h[d], L, inv);
+        } else {
             for (int d = 0; d < 3; d++) h[d] /= L;
         }
         for (int d = 0; d < 3; d++) g_cr[d] = 0.5 * g_area * n[d] + h[d];

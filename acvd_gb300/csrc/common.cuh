@@ -166,16 +166,40 @@ ACVD_DEV float recip_rn(float x) {
     return __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
 }
 
+// Whether 2^-465 <= |b| < 2^465, read off the exponent: a comparison in FP64 runs on the pipe
+// that bounds the kernels that ask.  Never for infinities and NaN.
+ACVD_DEV unsigned exponent_of(double b) { return ((unsigned)__double2hiint(b) >> 20) & 0x7ffu; }
+ACVD_DEV bool divides_well(double b) { return exponent_of(b) - 558u < 930u; }
+
 // a / b in FP64 from inv = 1 / b, where several quotients share the divisor: the product
 // corrected by its residual (Markstein 1990), 3 operations on the FP64 pipe instead of about
-// 9.  Before the last rounding the result is within 2^-51 units in the last place of a / b,
-// so it is the correctly rounded quotient unless a / b lies that close to a rounding boundary
-// (no difference in the 2^32 quotients that the test draws); inv must be a normal number
-// and a / b in the normal range, or zero.
-ACVD_DEV double quotient(double a, double b, double inv) {
+// 9.  Where both hold divides_well(), the residual is exact and the quotient normal; before
+// the last rounding the result is then within 2^-51 units in the last place of a / b, so it
+// is the correctly rounded quotient unless a / b lies that close to a rounding boundary (no
+// difference in the 2^33 quotients that the test draws).  Of a = 0 it is 0, +0 for -0.
+ACVD_DEV double quotient_in_range(double a, double b, double inv) {
     const double q = a * inv;
     return fma(fma(-b, q, a), inv, q);
 }
+
+// the same for any a: b alone holds divides_well()
+ACVD_DEV double quotient(double a, double b, double inv) {
+    if (__double_as_longlong(a) << 1 == 0) return a * inv;
+    return divides_well(a) ? quotient_in_range(a, b, inv) : a / b;
+}
+
+// Over a run of numerators, zeros aside: whether all held divides_well(), asked once at the
+// end (four integer operations each; a branch at each of an inverse's 41 quotients cost the
+// curvature fits 4 %).
+struct QuotientRange {
+    unsigned least = ~0u, most = 0u;
+    ACVD_DEV void add(double a) {
+        const unsigned u = 2u * (unsigned)__double2hiint(a) + min((unsigned)__double2loint(a), 1u);   // 0 for zeros
+        least = __viaddmin_u32(u, ~0u, least);
+        most = max(most, u);
+    }
+    ACVD_DEV bool holds() const { return least >= (558u << 21) - 1u && most < (558u + 930u) << 21; }
+};
 
 // The sums of products of the energy tests, each operation named: with the contraction left
 // to the compiler, the same source gave other last bits in another kernel, and with them

@@ -13,7 +13,8 @@
 // 6 x 6 inverse: 5.3 ms for 524,288 vertices at that rate.  So
 //  * products that depend on the face only are formed once per face;
 //  * quotients by one divisor (five per face, 51 per inverse) share its reciprocal
-//    (quotient(): 3 operations instead of about 9);
+//    (3 operations instead of about 9; what each needs to equal the division is checked on the
+//    exponents, with integer operations, 0.1 % of the time);
 //  * finding the 3-ring, integer work in dependent loads, has kernels of its own at their own
 //    occupancy instead of idling the FP64 pipe in between: every vertex's fan of faces
 //    once, then the list of each vertex's ring, in chunks of kCurvChunk vertices.
@@ -34,13 +35,6 @@ constexpr int kCurvMaxVis = 96;   // vertices of rings 0..2
 constexpr int64_t kCurvChunk = 1 << 19;
 
 constexpr int kFitBatch = 4;
-
-// whether 1 / b and quotients of such numbers by b stay in the normal range: 2^-465 <= |b| <
-// 2^465, read off the exponent (a comparison in FP64 runs on the pipe that bounds it all)
-__device__ __forceinline__ bool divides_well(double b) {
-    return (((unsigned)__double2hiint(b) >> 20) & 0x7ffu) - 558u < 930u;
-}
-__device__ __forceinline__ bool divided_well(double a) { return divides_well(a) || __double_as_longlong(a) << 1 == 0; }
 
 // Faces of edge e: the first two faces, in increasing id, holding both of its
 // endpoints (the reference attaches faces to an edge in face order,
@@ -105,12 +99,12 @@ __device__ void curv_face_mass(const double p1[3], const double p2[3], const dou
     const double a2 = 0.25 * sqrt(fabs(4.0 * a * c - (a - b + c) * (a - b + c)));
     for (int i = 0; i < 3; i++) {
         const double t = a2 * (p1[i] + p2[i] + p3[i]);
-        bary[i] = 0.0 + (divided_well(t) ? quotient(t, 3.0, 1.0 / 3.0) : t / 3.0);
+        bary[i] = 0.0 + quotient(t, 3.0, 1.0 / 3.0);
     }
     area = 0.0 + a2;
     if (divides_well(area)) {
         const double inv = 1.0 / area;
-        for (int i = 0; i < 3; i++) bary[i] = divided_well(bary[i]) ? quotient(bary[i], area, inv) : bary[i] / area;
+        for (int i = 0; i < 3; i++) bary[i] = quotient(bary[i], area, inv);
     } else if (area > 0) {
         for (int i = 0; i < 3; i++) bary[i] /= area;
     }
@@ -126,7 +120,7 @@ __device__ void curv_normal(const double x1[3], const double x2[3], const double
     const double l = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
     if (divides_well(l)) {
         const double inv = 1.0 / l;
-        for (int k = 0; k < 3; k++) n[k] = divided_well(n[k]) ? quotient(n[k], l, inv) : n[k] / l;
+        for (int k = 0; k < 3; k++) n[k] = quotient(n[k], l, inv);
     } else if (l != 0.0) {
         n[0] /= l; n[1] /= l; n[2] /= l;
     }
@@ -300,11 +294,19 @@ __global__ void __launch_bounds__(kRingThreads) ring_faces_kernel(CurvMesh m, in
 
 // Inverse of the n x n matrix a by LU decomposition with partial pivoting
 // (Doolittle), one substitution per unit vector; 0 when a pivot is exactly zero.
-template <int N>
-__device__ int curv_lu_invert(const double a[N][N], double ai[N][N]) {
+// SHARED: a pivot's quotients share its reciprocal; -1 if one was out of that form's range.
+// (A zero may lose its sign there: it ends in sums that start from +0 or hold another term
+// that is not -0, where both zeros give the same.)
+template <int N, bool SHARED>
+__device__ __forceinline__ int curv_lu_invert_by(const double a[N][N], double ai[N][N]) {
     double lu[N][N], rec[N];
-    bool good[N];
+    QuotientRange range;
     int piv[N];
+    auto over_pivot = [&](double x, int k) {
+        if (!SHARED) return x / lu[k][k];
+        range.add(x);
+        return quotient_in_range(x, lu[k][k], rec[k]);
+    };
     for (int i = 0; i < N; i++)
         for (int j = 0; j < N; j++) lu[i][j] = a[i][j];
     for (int k = 0; k < N; k++) {
@@ -314,15 +316,16 @@ __device__ int curv_lu_invert(const double a[N][N], double ai[N][N]) {
             const double v = fabs(lu[i][k]);
             if (v > best) { best = v; p = i; }
         }
-        if (best == 0.0) return 0;
+        if (best == 0.0) return SHARED && !range.holds() ? -1 : 0;
         piv[k] = p;
         if (p != k)
             for (int j = 0; j < N; j++) { const double t = lu[k][j]; lu[k][j] = lu[p][j]; lu[p][j] = t; }
-        const double d = lu[k][k];
-        good[k] = divides_well(d);
-        rec[k] = 1.0 / d;
+        if (SHARED) {
+            range.add(lu[k][k]);
+            rec[k] = 1.0 / lu[k][k];
+        }
         for (int i = k + 1; i < N; i++) {
-            const double f = good[k] ? quotient(lu[i][k], d, rec[k]) : lu[i][k] / d;
+            const double f = over_pivot(lu[i][k], k);
             lu[i][k] = f;
             for (int j = k + 1; j < N; j++) lu[i][j] -= f * lu[k][j];
         }
@@ -336,11 +339,30 @@ __device__ int curv_lu_invert(const double a[N][N], double ai[N][N]) {
             for (int j = 0; j < i; j++) x[i] -= lu[i][j] * x[j];
         for (int i = N - 1; i >= 0; i--) {
             for (int j = i + 1; j < N; j++) x[i] -= lu[i][j] * x[j];
-            x[i] = good[i] ? quotient(x[i], lu[i][i], rec[i]) : x[i] / lu[i][i];
+            x[i] = over_pivot(x[i], i);
         }
         for (int i = 0; i < N; i++) ai[i][c] = x[i];
     }
-    return 1;
+    return SHARED && !range.holds() ? -1 : 1;
+}
+
+template <int N>
+__device__ __noinline__ int curv_lu_invert_plain(const double a[N][N], double ai[N][N]) {
+    return curv_lu_invert_by<N, false>(a, ai);
+}
+
+template <int N>
+__device__ int curv_lu_invert(const double a[N][N], double ai[N][N]) {
+    const int r = curv_lu_invert_by<N, true>(a, ai);
+    if (r >= 0) return r;
+    // copies, so that the common case's matrices need no address
+    double b[N][N], bi[N][N];
+    for (int i = 0; i < N; i++)
+        for (int j = 0; j < N; j++) b[i][j] = a[i][j];
+    const int t = curv_lu_invert_plain<N>(b, bi);
+    for (int i = 0; i < N; i++)
+        for (int j = 0; j < N; j++) ai[i][j] = bi[i][j];
+    return t;
 }
 
 // Eigen-decomposition of the symmetric 2x2 matrix given by the upper triangle of
@@ -452,15 +474,21 @@ __device__ double curv_fit(const CurvMesh& m, const int* fl, int64_t stride, int
         xyt[i] = 0.0;
         for (int j = 0; j < 6; j++) xxt[i][j] = 0.0;
     }
+    // The quotients by h and h^2 share reciprocals.  |x| and |y| are at most nf h: for h in
+    // [2^-120, 2^120) and |x y| from 2^-250 on, both are 2^-378 or more, their squares and the
+    // quotients normal numbers and the residuals exact.  Other values that are zero, or so small
+    // or large, are looked at one by one.
     const double hh = h * h;
-    const bool good = divides_well(hh) && divides_well(h);
+    const bool good = divides_well(hh) && divides_well(h), near_one = exponent_of(h) - 903u < 240u;
     const double rh = 1.0 / h, rhh = 1.0 / hh;
+    auto squares_well = [](double v) { return exponent_of(v) - 791u < 464u || __double_as_longlong(v) << 1 == 0; };
     for (int k = 0; k < nf; k++) {
         const double x = xs[k], y = ys[k], z = zs[k];
         double r[6] = {1.0, x, y, x * x, x * y, y * y};
-        if (good) {
-            r[1] = quotient(r[1], h, rh); r[2] = quotient(r[2], h, rh);
-            r[3] = quotient(r[3], hh, rhh); r[4] = quotient(r[4], hh, rhh); r[5] = quotient(r[5], hh, rhh);
+        if ((near_one && exponent_of(r[4]) >= 773u) || (good && squares_well(x) && squares_well(y))) {
+            r[1] = quotient_in_range(x, h, rh); r[2] = quotient_in_range(y, h, rh);
+            r[3] = quotient_in_range(r[3], hh, rhh); r[4] = quotient_in_range(r[4], hh, rhh);
+            r[5] = quotient_in_range(r[5], hh, rhh);
         } else {
             r[1] /= h; r[2] /= h; r[3] /= hh; r[4] /= hh; r[5] /= hh;
         }
@@ -505,9 +533,11 @@ __device__ double curv_fit(const CurvMesh& m, const int* fl, int64_t stride, int
 
 // The fits of vertices v0 .. v0 + n - 1 over their face lists.  A neighbourhood that was too
 // large leaves the vertex's outputs at zero.  One warp per block: the SMs differ by a warp.
+// At least 12 of them to an SM: 204 registers otherwise, and 524,288 vertices took 7.81 ms
+// instead of 7.73.
 constexpr int kFitThreads = 32;
 
-__global__ void __launch_bounds__(kFitThreads) curvature_kernel(CurvMesh m, int64_t v0, int64_t n,
+__global__ void __launch_bounds__(kFitThreads, 12) curvature_kernel(CurvMesh m, int64_t v0, int64_t n,
                                                                 const int* __restrict__ lists,
                                                                 const int* __restrict__ counts,
                                                                 double* __restrict__ indicator,

@@ -189,7 +189,7 @@ ACVD_DEV double quotient(double a, double b, double inv) {
 }
 
 // Over a run of numerators, zeros aside: whether all held divides_well(), asked once at the
-// end (four integer operations each; a branch at each of an inverse's 41 quotients cost the
+// end (four integer operations each; a branch at each of an inverse's 51 quotients cost the
 // curvature fits 4 %).
 struct QuotientRange {
     unsigned least = ~0u, most = 0u;

@@ -17,7 +17,7 @@
 //    exponents, with integer operations, 0.1 % of the time);
 //  * finding the 3-ring, integer work in dependent loads, has kernels of its own at their own
 //    occupancy instead of idling the FP64 pipe in between: every vertex's fan of faces
-//    once, then the list of each vertex's ring, in chunks of kCurvChunk vertices.
+//    once, then the list of each vertex's ring, in chunks of curv_chunk() vertices.
 // 6.46 ms of fits and 0.76 of lists for 524,288 vertices; one kernel for both, with 8,500 FP64
 // operations per vertex, took 9.9 ms with its pipe 72 % busy.
 #include "../../include/acvd_gpu.h"
@@ -30,10 +30,6 @@ namespace acvd {
 constexpr int kCurvMaxF = 192;    // faces of one 3-ring
 constexpr int kCurvMaxV = 384;    // vertices queued for one ring step
 constexpr int kCurvMaxVis = 96;   // vertices of rings 0..2
-// vertices whose face lists are held at a time (up to 403 MB): enough blocks for the last
-// wave not to show
-constexpr int64_t kCurvChunk = 1 << 19;
-
 constexpr int kFitBatch = 4;
 
 // Faces of edge e: the first two faces, in increasing id, holding both of its
@@ -558,34 +554,38 @@ __global__ void __launch_bounds__(kFitThreads, 12) curvature_kernel(CurvMesh m, 
 
 static inline unsigned cgrid(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
-// Work of launch_curvature: the faces' values, the items' fans and the lists of a chunk.
-static int64_t curv_chunk(int64_t nv) { return nv < kCurvChunk ? nv : kCurvChunk; }
+// Vertices whose face lists are held at a time.  (Chunks of equal size instead of full ones
+// and a rest: 1024 x 513 the same 7.87 ms, 1024 x 1000 15.1 ms instead of 14.9: what counts is
+// how full the last wave of fits is, and 524,288 vertices are 8.98 waves of 12 warps to an SM.)
+static int64_t curv_chunk(int64_t nv, int64_t most) { return nv < most ? nv : most; }
 
-size_t curvature_work_bytes(int64_t nv, int64_t nf, int64_t ne) {
+// Work of launch_curvature: the faces' values, the items' fans and the lists of a chunk.
+size_t curvature_work_bytes(int64_t nv, int64_t nf, int64_t ne, int64_t most) {
     return (size_t)nf * sizeof(FaceProps) +
-           sizeof(int) * (size_t)(4 * ne + nv + curv_chunk(nv) * (kCurvMaxF + 1));
+           sizeof(int) * (size_t)(4 * ne + nv + curv_chunk(nv, most) * (kCurvMaxF + 1));
 }
 
 cudaError_t launch_curvature(const double* xyz, const int* tri, int64_t nv, int64_t nf, int64_t ne,
                              const int* edge_v, const int* edge_int, const uint32_t* vf_row, const uint32_t* vf_face,
                              const int* row, const int* col, const int* inv, int2* poly, int* slot_edge, void* work,
-                             double* indicator, float* dirs, unsigned long long* overflow, cudaStream_t s) {
+                             int64_t most, double* indicator, float* dirs, unsigned long long* overflow, cudaStream_t s) {
     if (nv == 0) return cudaSuccess;
     cudaError_t err = cudaMemsetAsync(slot_edge, 0xff, 2 * ne * sizeof(int), s);   // -1: no edge
     if (err != cudaSuccess) return err;
     g_launches += 4;
     FaceProps* fp = (FaceProps*)work;
+    const int64_t chunk = curv_chunk(nv, most);
     int* fan = (int*)(fp + nf);
     int* fan_count = fan + 4 * ne;
     int* counts = fan_count + nv;
-    int* lists = counts + curv_chunk(nv);
+    int* lists = counts + chunk;
     face_props_kernel<<<cgrid(nf, 256), 256, 0, s>>>(xyz, tri, nf, fp);
     edge_faces_kernel<<<cgrid(ne, 256), 256, 0, s>>>(edge_v, ne, tri, vf_row, vf_face, poly);
     slot_edges_kernel<<<cgrid(ne, 256), 256, 0, s>>>(edge_int, ne, row, col, slot_edge);
     fan_kernel<<<cgrid(nv, 256), 256, 0, s>>>(nv, row, slot_edge, poly, fan, fan_count);
     const CurvMesh m{fp, nv, row, col, inv, fan, fan_count};
-    for (int64_t v0 = 0; v0 < nv; v0 += kCurvChunk) {
-        const int64_t n = nv - v0 < kCurvChunk ? nv - v0 : kCurvChunk;
+    for (int64_t v0 = 0; v0 < nv; v0 += chunk) {
+        const int64_t n = nv - v0 < chunk ? nv - v0 : chunk;
         g_launches += 2;
         ring_faces_kernel<<<cgrid(n, kRingGroups), kRingThreads, 0, s>>>(m, v0, n, lists, counts, overflow);
         curvature_kernel<<<cgrid(n, kFitThreads), kFitThreads, 0, s>>>(m, v0, n, lists, counts, indicator, dirs);

@@ -1780,6 +1780,11 @@ extern "C" int acvd_get_boundary_edges(acvd_ctx* ctx, int32_t* ids, int64_t* cou
     return ACVD_OK;
 }
 
+// The work of a curvature call stays with the context: 80 bytes per face, 16 per edge, 4 per
+// vertex, and the face lists of at most this many vertices at a time (ACVD_CURV_CHUNK), 772
+// bytes each, up to 405 MB: enough blocks for the last wave of a chunk not to show.
+constexpr int64_t kDefaultCurvChunk = 1 << 19;
+
 // Curvature of vertex clustering (vtkDiscreteRemeshing.h:630-637 ->
 // vtkCurvatureMeasure, polynomial fitting on the vertex 3-ring): indicator[nV]
 // and principal_dirs[6 nV], either may be NULL.
@@ -1795,10 +1800,12 @@ extern "C" int acvd_compute_curvature(acvd_ctx* ctx, double* indicator, float* p
     CK(ctx->dtmp.resize(2));
     unsigned long long* overflow = (unsigned long long*)ctx->dtmp.p;
     CK(cudaMemsetAsync(overflow, 0, sizeof(unsigned long long), ctx->s));
-    CK(ctx->curv_work.resize(curvature_work_bytes(nv, ctx->nF, ne)));
+    int64_t most = kDefaultCurvChunk;
+    if (const char* e = std::getenv("ACVD_CURV_CHUNK")) most = std::max<int64_t>(1, std::atoll(e));
+    CK(ctx->curv_work.resize(curvature_work_bytes(nv, ctx->nF, ne, most)));
     CK(launch_curvature(ctx->xyz.p, ctx->tri.p, nv, ctx->nF, ne, ctx->edge_v.p, ctx->edge_int.p, ctx->vf_row.p,
                         ctx->vf_face.p, ctx->row.p, ctx->col.p, ctx->inv.p, ctx->curv_poly.p, ctx->curv_slot.p,
-                        ctx->curv_work.p, ctx->curv_ind.p, ctx->curv_dirs.p, overflow, ctx->s));
+                        ctx->curv_work.p, most, ctx->curv_ind.p, ctx->curv_dirs.p, overflow, ctx->s));
     unsigned long long h_over = 0;
     CK(cudaMemcpyAsync(&h_over, overflow, sizeof h_over, cudaMemcpyDeviceToHost, ctx->s));
     if (indicator)

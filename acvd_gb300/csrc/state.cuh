@@ -412,12 +412,13 @@ cudaError_t launch_boundary_edges(const int* edge_v, int64_t ne, const int* labe
                                   uint32_t* scratch, size_t scratch_words, cudaStream_t s);
 
 // ---- curvature (curvature.cu) ----
-// work: curvature_work_bytes, 8-byte aligned; poly: ne, slot_edge: 2 ne
-size_t curvature_work_bytes(int64_t nv, int64_t nf, int64_t ne);
+// most: vertices whose face lists may be held at a time; work: curvature_work_bytes, 8-byte
+// aligned; poly: ne, slot_edge: 2 ne
+size_t curvature_work_bytes(int64_t nv, int64_t nf, int64_t ne, int64_t most);
 cudaError_t launch_curvature(const double* xyz, const int* tri, int64_t nv, int64_t nf, int64_t ne,
                              const int* edge_v, const int* edge_int, const uint32_t* vf_row, const uint32_t* vf_face,
                              const int* row, const int* col, const int* inv, int2* poly, int* slot_edge, void* work,
-                             double* indicator, float* dirs, unsigned long long* overflow, cudaStream_t s);
+                             int64_t most, double* indicator, float* dirs, unsigned long long* overflow, cudaStream_t s);
 
 // ---- midpoint subdivision (subdivide.cu) ----
 // One level of vtkSurface::Subdivide over a mesh in the reference's numbering

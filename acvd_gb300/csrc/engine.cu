@@ -1310,8 +1310,8 @@ static bool use_cluster(acvd_ctx* ctx) {
 
 // Runs colour sweeps on the device until the host loop's convergence test is
 // met: one cooperative launch, or (cluster) launches of one cluster, which return after
-// kClusterRun sweeps at most.  hl carries the loop state in and out.
-constexpr int kClusterRun = 4096;
+// kDefaultClusterRun sweeps at most (ACVD_CLUSTER_RUN).  hl carries the loop state in and out.
+constexpr int kDefaultClusterRun = 4096;
 
 static int run_sweeps_persistent(acvd_ctx* ctx, LoopState& hl, acvd_stats& local, bool cluster) {
     const int grid = cluster ? kClusterCtas : sweep_run_grid(ctx);
@@ -1343,7 +1343,8 @@ static int run_sweeps_persistent(acvd_ctx* ctx, LoopState& hl, acvd_stats& local
     a.log = ctx->slog.p;
     a.log_cap = kSweepLogCap;
     if (cluster) {
-        a.max_run = kClusterRun;
+        a.max_run = kDefaultClusterRun;
+        if (const char* e = std::getenv("ACVD_CLUSTER_RUN")) a.max_run = std::max(1, std::atoi(e));
         do {
             CK(launch_sweep_cluster(ctx->metric, a, ctx->s));
             CK(cudaMemcpyAsync(&hl, ctx->dls.p, sizeof hl, cudaMemcpyDeviceToHost, ctx->s));

@@ -1297,10 +1297,15 @@ static int sweep_run_grid(acvd_ctx* ctx) {
 //   isotropic   2084 / 1873  2240 / 2012  2803 / 2720  3498 / 4033
 //   QEM         3273 / 2879  5545 / 5167  5828 / 6469  6601 / 8989
 //   anisotropic 3995 / 3552  8260 / 7705  7381 / 8264  9124 / 12517
+// With K = items / 60, / 8 and / 3 the cluster is 4 to 25 % faster for 2,560 to 12,672 items
+// too, but for the anisotropic metric at 12,672 items and K = items / 3 (4466 / 4538).  More
+// clusters than items leave passes over empty clusters, on 16 SMs (K = 64 items: 1 to 4 %
+// slower than the graph): those stay with the graph.
 constexpr int64_t kDefaultClusterMax = 3072;
 
 static bool use_cluster(acvd_ctx* ctx) {
     if (ctx->has_work) return false;   // split classes asked for (ACVD_SPLIT_MIN): their two kernels
+    if (ctx->K > ctx->nV) return false;
     int64_t most = 0;
     for (int c = 0; c < ctx->nclasses; c++) most = std::max(most, ctx->sweep_off[c + 1] - ctx->sweep_off[c]);
     int64_t limit = kDefaultClusterMax;

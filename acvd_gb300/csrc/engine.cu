@@ -125,6 +125,7 @@ struct acvd_ctx {
     int* h_color = nullptr;                    // pinned colours of the host colourings
     int64_t h_color_cap = 0;
     unsigned long long h_counters[kNumCounters] = {};   // stripes summed
+    unsigned long long at_connexity[kNumCounters] = {};   // those when the connectivity constraint began
     DBuf<RunFlags> dflags;
     RunFlags flags{1, 0, 3, 1e-3f};
     int level = 3;
@@ -1394,14 +1395,19 @@ static int energy_total(acvd_ctx* ctx, double* out) {
 // item its boundary flag; per screened item its 8-slot ring, label and evaluation
 // sweep; per ring slot the neighbour's label; per cached screen its 16-byte record
 // (cluster, targets, evaluation sweep) and up to 4 cluster stamps; per boundary item its record, its
-// cluster's record and size; per destination cluster its record; per proposal the
-// candidate slots and two claim words.
+// cluster's record and size; per destination cluster its record; per proposal its 16-byte record
+// and the source's 4-byte count of leavers, read and written.  Under the connectivity
+// constraint also the packed ring adjacency (8) per screened item, and per proposal two
+// 8-byte claims in the count's place.
 static int64_t eval_bytes_of(const acvd_ctx* ctx, const unsigned long long* c) {
     const int64_t R = ctx->metric == kIso ? 16 : (ctx->metric == kQEM ? 40 : 64);
     const int64_t C = 16 * (int64_t)ev_stride(ctx->metric);
+    int64_t constrained = 0;
+    if (ctx->flags.connexity)
+        for (int q : {kCntScreened, kCntCand}) constrained += (int64_t)(c[q] - ctx->at_connexity[q]);
     return 1 * (int64_t)c[kCntVisited] + 40 * (int64_t)c[kCntScreened] + 32 * (int64_t)c[kCntCached] +
            4 * (int64_t)c[kCntSlots] + (R + C + 4) * (int64_t)c[kCntBoundary] + C * (int64_t)c[kCntTargets] +
-           24 * (int64_t)c[kCntCand];
+           24 * (int64_t)c[kCntCand] + 8 * constrained;
 }
 
 // the per-sweep log's snapshot of the cumulative counters
@@ -1627,6 +1633,7 @@ extern "C" int acvd_minimize(acvd_ctx* ctx, acvd_stats* stats) {
                 }
                 if (convergences >= 1 && !ctx->flags.connexity) {
                     ctx->flags.connexity = 1;
+                    std::copy(ctx->h_counters, ctx->h_counters + kNumCounters, ctx->at_connexity);
                     flags_changed = true;
                 }
                 if (slog.f) {

@@ -11,7 +11,7 @@ Two families of candidates:
 * exact schedules give the default schedule's clustering bit for bit, so a tuned run never
   changes a result:
     - ``graphs``: per-phase kernels, sweeps between convergence events looped on the device
-      inside one CUDA graph (the default);
+      inside one CUDA graph, or, for small meshes, in one thread-block cluster (the default);
     - ``host_loop``: the same kernels, one graph launch per sweep decided on the host;
     - ``persistent``: one cooperative kernel per phase with grid barriers;
     - ``fused``: the launch shape of the evaluation -- every colour class through the one
@@ -21,8 +21,9 @@ Two families of candidates:
       blocks of 256 threads per SM (80, 64 or 48 registers per thread) instead of the
       per-kernel defaults;
     - ``threads128``: the evaluation kernels in blocks of 128 threads (8 per SM, 64
-      registers; the default shape): a block waits at its tile's barriers, and smaller blocks let more of them
-      be in different phases.
+      registers), by name: a block waits at its tile's barriers, and smaller blocks let more
+      of them be in different phases.  The default has this shape, so the two measure equal;
+      the name stays for the caches that hold it.
   A candidate of this family whose labels differ from the default's is rejected, since that
   would mean a broken guarantee rather than a faster schedule.
 * approximate schedules (opt-in) reach a different deterministic clustering:

@@ -771,24 +771,25 @@ ACVD_DEV void eval_tile(const DevState& st, int item0, int64_t count, int color,
     }
 }
 
-// The evaluation kernels are compiled for 3, 4 and 5 blocks of 256 threads per SM
-// (registers per thread follow: 3 -> 80, 4 -> 64, 5 -> 48): fewer blocks spill
-// less of the energy tests, more hide more latency, and which wins depends on the
-// metric and the workload.  launch_eval takes the count at run time (the context's
-// eval_blocks, ACVD_EVAL_BLOCKS; the autotuner times the choices); 0 selects the
-// defaults below, measured on GB300.
 // TB: threads (and items) per block.  A block is the unit that waits at the tile's
 // barriers, so smaller blocks at the same threads per SM (B * 256 / TB blocks of TB)
-// let more of them be in different phases of their tiles.
+// let more of them be in different phases of their tiles: the default is 128 threads, 8
+// blocks per SM (64 registers a thread), for every metric.  Blocks of 256 are compiled for
+// 3, 4 and 5 per SM (80, 64 and 48 registers: fewer spill less of the energy tests, more
+// hide more latency); launch_eval takes the context's eval_blocks and eval_threads
+// (ACVD_EVAL_BLOCKS, ACVD_EVAL_THREADS; the autotuner times the choices).  Converged solves in
+// ms, 256 threads at 3 / 4 / 5 blocks, 128 threads: 1024 x 512 quadric torus 11.13 / 10.95 / 11.01,
+// 10.64 to 10.94; 4096^2 anisotropic heightfield 181.0 / 171.4 / 177.1, 173.2; batch of 256 quadric
+// meshes 100.2 / 96.5 / 96.2, 97.1.
 template <int M, int B, int TB = 256>
 __global__ void __launch_bounds__(TB, B * 256 / TB) eval_kernel(DevState st, int item0, int64_t count, int color,
                                                                 int claims, int per) {
     eval_tile<M, TB>(st, item0, count, color, claims, blockIdx.x, per);
 }
 
-// default blocks per SM: the fused evaluation 4 (isotropic, QEM) and 5 (the
-// quadric-anisotropic metric: 330 ms against 347 ms on the 4096^2 heightfield when it
-// ran every class); the work-list evaluation 4 (222 ms against 232 at 3 and 241 at 5)
+// blocks of 256 per SM where only ACVD_EVAL_THREADS=256 was asked for: the fused evaluation 4
+// (isotropic, QEM) and 5 (the quadric-anisotropic metric, by which it was faster when every
+// class ran it), the work-list evaluation 4
 constexpr int default_eval_blocks(int metric) { return metric == kAniso ? 5 : 4; }
 constexpr int kDefaultListBlocks = 4;
 

@@ -327,7 +327,7 @@ def run_subdivision_arm(args):
                "d2h_bytes_per_step": int(out[0].nbytes + out[1].nbytes + out[2].nbytes + out[3].nbytes +
                                          out[4].nbytes),
                "ms_per_step": statistics.mean(e2e_ms),
-               "includes": "host->device inputs, the three kernels, device->host outputs (pageable results)"}
+               "includes": "host->device inputs, the kernels, device->host outputs (pageable results)"}
     eng.close()
     if rank != 0:
         return
@@ -356,7 +356,7 @@ def run_subdivision_arm(args):
         "vs_baseline": None, "dtype": "f64", "data": "synthetic",
         "config": {"workload": args.workload, "description": w["desc"], "vertices": nv, "edges": ne, "faces": nf,
                    "l2": "flushed between timed steps (256 MB write)"},
-        "roofline": {"bound": "hbm", "kernel": "subdiv_* (three kernels and a memset, timed together)",
+        "roofline": {"bound": "hbm", "kernel": "subdiv_* (two kernels and a memset, timed together)",
                      "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else "fallback",
                      "traffic": None, "algorithmic_bytes_per_launch": alg},
